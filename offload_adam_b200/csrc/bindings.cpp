@@ -435,6 +435,7 @@ struct PyEngine {
 
 }  // namespace
 
+void bind_loss(py::module_& m);
 void bind_quant(py::module_& m);
 void bind_symm(py::module_& m);
 
@@ -535,6 +536,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("bytes_d2h", &PyEngine::bytes_d2h)
       .def("reset_counters", &PyEngine::reset_counters);
 
+  bind_loss(m);
   bind_quant(m);
   bind_symm(m);
 }

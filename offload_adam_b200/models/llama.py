@@ -24,6 +24,9 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
 
+from .. import _ext
+from ..ops.dispatch import use_kernels
+
 
 @dataclass
 class LlamaConfig:
@@ -153,10 +156,10 @@ class DecoderLayer(nn.Module):
 
 
 class _ChunkedLinearCE(torch.autograd.Function):
-    """mean cross-entropy of ``h @ W^T`` against ``labels`` (ignore_index=-100),
-    computed chunk by chunk.  Gradients with respect to ``h`` and ``W`` are formed
-    in the same pass and only scaled in backward, so the logits of a chunk are
-    live for one chunk only."""
+    """mean cross-entropy of ``h @ W^T`` against ``labels`` (ignore_index=-100), in the
+    operations of PyTorch, chunk by chunk.  Gradients with respect to ``h`` and ``W`` are
+    formed in the same pass and only scaled in backward, so the logits of a chunk are live
+    for one chunk only."""
 
     @staticmethod
     def forward(ctx, h, weight, labels, chunk):
@@ -191,7 +194,95 @@ class _ChunkedLinearCE(torch.autograd.Function):
         return gh * g.to(gh.dtype), gw * g.to(gw.dtype), None, None
 
 
+# Rows of the logits that the kernel route handles at a time, in units of the caller's chunk.
+# The torch route holds a chunk's logits in bf16 and fp32, its probabilities in fp32 and their
+# bf16 image, 12 bytes an element, next to an fp32 gradient of the head; the kernel route holds
+# bf16 logits and, in backward, their bf16 gradient: 4 bytes for up to three times the rows.
+_CE_ROWS_PER_CHUNK = 3
+
+
+class _KernelLinearCE(torch.autograd.Function):
+    """The same loss through ``csrc/loss_ops.cu`` (bf16, CUDA).
+
+    Up to ``_CE_ROWS_PER_CHUNK`` chunks of rows: forward keeps the bf16 logits and two floats
+    a row; backward turns them into the gradient of the logits, the incoming gradient
+    folded in, and both matrix products run once over all rows, accumulating in fp32.
+    More rows than that: gradients are formed in forward, a group of rows at a time, and
+    scaled in backward."""
+
+    @staticmethod
+    def forward(ctx, h, weight, labels, chunk):
+        C = _ext.load(required=True)
+        N, V = h.shape[0], weight.shape[0]
+        f32 = dict(dtype=torch.float32, device=h.device)
+        loss, inv = torch.empty((), **f32), torch.empty((), **f32)
+        ctx.want_grad = ctx.needs_input_grad[0] or ctx.needs_input_grad[1]
+        rows = chunk * _CE_ROWS_PER_CHUNK
+        ctx.one_group = N <= rows
+        logits = C.ce_logits_buffer(h, min(N, rows), V)
+        stats = torch.empty(3 * logits.shape[0], **f32)
+        if ctx.one_group:
+            torch.mm(h, weight.T, out=logits)
+            C.ce_stats(logits, labels, stats)
+            C.ce_finish(stats[2 * N:], labels, loss, inv)
+            if ctx.want_grad:
+                ctx.save_for_backward(h, weight, labels, logits, stats, inv)
+            return loss
+        row_loss = torch.empty(N, **f32)
+        if ctx.want_grad:
+            C.ce_finish(None, labels, None, inv)
+            gh = torch.empty_like(h)
+            gw = torch.zeros(weight.shape, **f32)
+        for s in range(0, N, rows):
+            n = min(N - s, rows)
+            hs, lab, lo, st = h[s:s + n], labels[s:s + n], logits[:n], stats[:3 * n]
+            torch.mm(hs, weight.T, out=lo)
+            C.ce_stats(lo, lab, st)
+            row_loss[s:s + n] = st[2 * n:]
+            if ctx.want_grad:
+                C.ce_grad(lo, lab, st, inv, None, lo)
+                torch.mm(lo, weight, out=gh[s:s + n])
+                gw.add_(lo.T @ hs)
+        C.ce_finish(row_loss, labels, loss, inv)
+        if ctx.want_grad:
+            ctx.save_for_backward(gh, gw.to(weight.dtype))
+        return loss
+
+    @staticmethod
+    def backward(ctx, g):
+        if not ctx.one_group:
+            gh, gw = ctx.saved_tensors
+            return gh * g.to(gh.dtype), gw * g.to(gw.dtype), None, None
+        C = _ext.load(required=True)
+        h, weight, labels, logits, stats, inv = ctx.saved_tensors
+        through = g.requires_grad and torch.is_grad_enabled()  # keep the graph through g
+        # saved-tensor hooks may have returned copies without the padded rows
+        if logits.stride(0) % 16 or logits.data_ptr() % 32 or not _whole_vectors(logits):
+            logits = C.ce_logits_buffer(logits, *logits.shape).copy_(logits)
+        d = C.ce_logits_buffer(logits, *logits.shape)
+        with torch.no_grad():
+            C.ce_grad(logits, labels, stats, inv, None if through else g.detach().float().contiguous(), d)
+            gh = d @ weight if ctx.needs_input_grad[0] else None
+            gw = d.T @ h if ctx.needs_input_grad[1] else None
+        if through:
+            gh = None if gh is None else gh * g.to(gh.dtype)
+            gw = None if gw is None else gw * g.to(gw.dtype)
+        return gh, gw, None, None
+
+
+def _whole_vectors(x):
+    """True when every row of the 2-D view ``x``, the last one too, can be read up to the
+    next multiple of 16 elements without leaving the storage."""
+    end = x.storage_offset() + (x.shape[0] - 1) * x.stride(0) + (x.shape[1] + 15) // 16 * 16
+    return x.stride(1) == 1 and end * x.element_size() <= x.untyped_storage().nbytes()
+
+
 def chunked_linear_cross_entropy(h, weight, labels, chunk=2048):
+    kernels = (use_kernels(h, weight) and h.dim() == 2 and weight.dim() == 2 and h.numel() > 0 and weight.numel() > 0
+               and type(labels) is torch.Tensor and labels.is_cuda and labels.dtype == torch.int64
+               and labels.shape == h.shape[:1] and h.device == weight.device == labels.device)
+    if kernels:
+        return _KernelLinearCE.apply(h, weight, labels.contiguous(), chunk)
     return _ChunkedLinearCE.apply(h, weight, labels, chunk)
 
 
