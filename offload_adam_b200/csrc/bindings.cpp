@@ -436,6 +436,7 @@ struct PyEngine {
 }  // namespace
 
 void bind_loss(py::module_& m);
+void bind_model(py::module_& m);
 void bind_quant(py::module_& m);
 void bind_symm(py::module_& m);
 
@@ -537,6 +538,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("reset_counters", &PyEngine::reset_counters);
 
   bind_loss(m);
+  bind_model(m);
   bind_quant(m);
   bind_symm(m);
 }

@@ -1,0 +1,120 @@
+// Autograd functions of the elementwise model kernels and their Python bindings.  The
+// graph nodes are C++ so that a call costs the host about what one PyTorch operation does.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include "model_ops.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+namespace {
+
+cudaStream_t cur() { return at::cuda::getCurrentCUDAStream().stream(); }
+void ok(cudaError_t e, const char* what) { TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e)); }
+void check_bf16(const Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16, name, " must be a bf16 CUDA tensor");
+}
+
+// --------------------------------------------------------------------- SwiGLU
+struct SwiGLU : torch::autograd::Function<SwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& g, const Tensor& u) {
+    check_bf16(g, "gate");
+    check_bf16(u, "up");
+    TORCH_CHECK(g.sizes() == u.sizes() && g.device() == u.device(), "gate and up must have one shape and device");
+    c10::cuda::CUDAGuard guard(g.device());
+    const Tensor gc = g.contiguous(), uc = u.contiguous();
+    Tensor y = at::empty_like(gc);
+    ok(oab::launch_swiglu(gc.data_ptr(), uc.data_ptr(), y.data_ptr(), y.numel(), cur()), "swiglu");
+    ctx->save_for_backward({g, u});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &g = saved[0], &u = saved[1], &gy = grads[0];
+    if (!gy.defined()) return {Tensor(), Tensor()};
+    if (at::GradMode::is_enabled()) {  // a graph of the gradient is asked for
+      const Tensor s = at::sigmoid(g);
+      return {gy * u * s * (1 + g * (1 - s)), gy * at::silu(g)};
+    }
+    c10::cuda::CUDAGuard guard(g.device());
+    const Tensor c = gy.to(at::kBFloat16).contiguous(), gc = g.contiguous(), uc = u.contiguous();
+    Tensor gg = at::empty_like(gc), gu = at::empty_like(uc);
+    ok(oab::launch_swiglu_grad(c.data_ptr(), gc.data_ptr(), uc.data_ptr(), gg.data_ptr(), gu.data_ptr(), gc.numel(), cur()),
+       "swiglu_grad");
+    return {gg, gu};
+  }
+};
+
+// ----------------------------------------------------------------------- RoPE
+// (batch, seq, heads, dim) with unit stride along dim and 16-byte aligned heads
+Tensor rope_layout(const Tensor& x) {
+  const bool fits = x.stride(3) == 1 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 && x.stride(2) % 8 == 0 &&
+                    (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
+  return fits ? x : x.clone(at::MemoryFormat::Contiguous);
+}
+oab::RopeTensor rope_arg(const Tensor& x, const Tensor& y) {
+  oab::RopeTensor t;
+  if (!x.defined()) return t;
+  t.in = x.data_ptr();
+  t.out = y.data_ptr();
+  t.sb = x.stride(0);
+  t.ss = x.stride(1);
+  t.sh = x.stride(2);
+  t.heads = (int)x.size(2);
+  return t;
+}
+// either of q, k may be undefined
+variable_list rope_run(const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin, bool transposed) {
+  const Tensor& any = q.defined() ? q : k;
+  if (!any.defined()) return {Tensor(), Tensor()};
+  c10::cuda::CUDAGuard guard(any.device());
+  const Tensor qi = q.defined() ? rope_layout(q) : q, ki = k.defined() ? rope_layout(k) : k;
+  const Tensor qo = q.defined() ? at::empty(q.sizes(), q.options()) : q;
+  const Tensor ko = k.defined() ? at::empty(k.sizes(), k.options()) : k;
+  ok(oab::launch_rope(rope_arg(qi, qo), rope_arg(ki, ko), cos.data_ptr(), sin.data_ptr(), any.size(0), any.size(1),
+                      (int)any.size(3), transposed, cur()), "rope");
+  return {qo, ko};
+}
+Tensor rope_grad_graph(const Tensor& g, const Tensor& cos, const Tensor& sin) {
+  if (!g.defined()) return g;
+  const int64_t half = g.size(3) / 2;
+  const Tensor z = g * sin.unsqueeze(1);
+  return g * cos.unsqueeze(1) + at::cat({z.narrow(3, half, half), -z.narrow(3, 0, half)}, 3);
+}
+
+struct Rope : torch::autograd::Function<Rope> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
+    check_bf16(q, "q");
+    check_bf16(k, "k");
+    check_bf16(cos, "cos");
+    check_bf16(sin, "sin");
+    TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && q.size(0) == k.size(0) && q.size(1) == k.size(1) &&
+                    q.size(3) == k.size(3) && q.size(3) % 16 == 0, "rope: (batch, seq, heads, dim), dim % 16 == 0");
+    TORCH_CHECK(cos.dim() == 2 && cos.sizes() == sin.sizes() && cos.size(0) == q.size(1) && cos.size(1) == q.size(3) &&
+                    cos.is_contiguous() && sin.is_contiguous(), "rope: contiguous (seq, dim) tables");
+    ctx->set_materialize_grads(false);  // either head tensor may go unused
+    ctx->save_for_backward({cos, sin});
+    return rope_run(q, k, cos, sin, false);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    if (at::GradMode::is_enabled())
+      return {rope_grad_graph(grads[0], saved[0], saved[1]), rope_grad_graph(grads[1], saved[0], saved[1]), Tensor(), Tensor()};
+    auto out = rope_run(grads[0], grads[1], saved[0], saved[1], true);
+    return {out[0], out[1], Tensor(), Tensor()};
+  }
+};
+
+}  // namespace
+
+void bind_model(py::module_& m) {
+  m.def("swiglu", [](const Tensor& g, const Tensor& u) { return SwiGLU::apply(g, u); });
+  m.def("rope", [](const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
+    auto out = Rope::apply(q, k, cos, sin);
+    return std::make_pair(out[0], out[1]);
+  });
+}

@@ -1,0 +1,29 @@
+// Host-side launch interface of the elementwise model kernels (model_ops.cu): bf16 in and
+// out, fp32 inside, one rounding per result.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace oab {
+
+// y = silu(g) * u
+cudaError_t launch_swiglu(const void* g, const void* u, void* y, int64_t n, cudaStream_t st);
+// gg = gy * u * silu'(g), gu = gy * silu(g)
+cudaError_t launch_swiglu_grad(const void* gy, const void* g, const void* u, void* gg, void* gu, int64_t n,
+                               cudaStream_t st);
+
+// A (batch, seq, heads, dim) tensor of bf16 with unit stride along dim; strides in elements.
+struct RopeTensor {
+  const void* in = nullptr;
+  void* out = nullptr;  // contiguous
+  int64_t sb = 0, ss = 0, sh = 0;
+  int heads = 0;
+};
+// Rotates the heads of q and k (either may have 0 heads) by the tables cos / sin
+// (seq, dim): out[i] = x[i] cos[i] - x[i + d/2] sin[i] for the first half of dim,
+// out[i] = x[i] cos[i] + x[i - d/2] sin[i] for the second; the transpose of that when
+// `transposed`.  dim % 16 == 0; bases and strides 16-byte aligned.
+cudaError_t launch_rope(const RopeTensor& q, const RopeTensor& k, const void* cos, const void* sin, int64_t batch,
+                        int64_t seq, int dim, bool transposed, cudaStream_t st);
+
+}  // namespace oab

@@ -123,10 +123,16 @@ class Attention(nn.Module):
         k = self.k_proj(x).view(B, S, self.nkv, self.hd)
         if self.q_norm is not None:
             q, k = self.q_norm(q), self.k_norm(k)
-        q, k = q.transpose(1, 2), k.transpose(1, 2)
         v = self.v_proj(x).view(B, S, self.nkv, self.hd).transpose(1, 2)
-        q = _apply_rope(q, cos, sin)
-        k = _apply_rope(k, cos, sin)
+        # heads in whole pairs of 8-value vectors, tables as _rope_for makes them
+        if (self.hd % 16 == 0 and use_kernels(q, k, cos, sin) and cos.shape == sin.shape == (S, self.hd)
+                and cos.is_contiguous() and sin.is_contiguous() and not (cos.requires_grad or sin.requires_grad)
+                and q.device == k.device == cos.device == sin.device):
+            q, k = _ext.load(required=True).rope(q, k, cos, sin)
+            q, k = q.transpose(1, 2), k.transpose(1, 2)
+        else:
+            q = _apply_rope(q.transpose(1, 2), cos, sin)
+            k = _apply_rope(k.transpose(1, 2), cos, sin)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.nh != self.nkv)
         return self.o_proj(o.transpose(1, 2).reshape(B, S, self.nh * self.hd))
 
@@ -139,7 +145,10 @@ class MLP(nn.Module):
         self.down_proj = nn.Linear(cfg.intermediate_size, cfg.hidden_size, bias=False)
 
     def forward(self, x):
-        return self.down_proj(F.silu(self.gate_proj(x)) * self.up_proj(x))
+        gate, up = self.gate_proj(x), self.up_proj(x)
+        if use_kernels(gate, up) and gate.shape == up.shape and gate.device == up.device:
+            return self.down_proj(_ext.load(required=True).swiglu(gate, up))
+        return self.down_proj(F.silu(gate) * up)
 
 
 class DecoderLayer(nn.Module):

@@ -1,0 +1,105 @@
+"""Elementwise model kernels against the same formulas in fp64 PyTorch."""
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from offload_adam_b200 import _ext
+from offload_adam_b200.models.llama import _apply_rope, _rope_tables, build_llama, tiny_llama
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, seed=0, std=1.0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=gen) * std).to(torch.bfloat16)
+
+
+def _close(got, want, slack=1.01):
+    """One rounding to bf16 (8 significant bits: 2^-8 of the value) on top of a few fp32 ulp."""
+    err = (got.double() - want).abs()
+    assert (err <= slack * 2.0 ** -8 * want.abs() + 1e-6 * want.abs().max() + 1e-37).all(), err.max().item()
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4096, 4097, 100003])
+def test_swiglu(n):
+    C = _ext.load(required=True)
+    g, u, gy = _rand(n, seed=1, std=4.0), _rand(n, seed=2), _rand(n, seed=3)
+    g[0] = -80.0
+    a, b = g.clone().requires_grad_(True), u.clone().requires_grad_(True)
+    y = C.swiglu(a, b)
+    y.backward(gy)
+    a64, b64 = g.double().requires_grad_(True), u.double().requires_grad_(True)
+    y64 = F.silu(a64) * b64
+    y64.backward(gy.double())
+    _close(y.detach(), y64.detach())
+    _close(a.grad, a64.grad)
+    _close(b.grad, b64.grad)
+
+
+def test_swiglu_views_and_second_derivative():
+    C = _ext.load(required=True)
+    base = _rand(64, 70, seed=4)
+    g, u = base[:, 1:33], base.t()[:64, :32].contiguous()[:, :32]
+    _close(C.swiglu(g, u), F.silu(g.double()) * u.double())
+    a = _rand(40, seed=5).requires_grad_(True)
+    b = _rand(40, seed=6)
+    d, = torch.autograd.grad(C.swiglu(a, b).float().sum(), a, create_graph=True)
+    dd, = torch.autograd.grad(d.float().sum(), a)
+    a64 = a.detach().double().requires_grad_(True)
+    d64, = torch.autograd.grad((F.silu(a64) * b.double()).sum(), a64, create_graph=True)
+    dd64, = torch.autograd.grad(d64.sum(), a64)
+    assert (dd.double() - dd64).norm() <= 2e-2 * dd64.norm()
+
+
+@pytest.mark.parametrize("dim", [16, 32, 64, 96, 128])
+@pytest.mark.parametrize("batch,seq,heads,kv", [(1, 1, 1, 1), (2, 17, 4, 2), (1, 300, 5, 5)])
+def test_rope(dim, batch, seq, heads, kv):
+    C = _ext.load(required=True)
+    cos, sin = (t.to(torch.bfloat16) for t in _rope_tables(seq, dim, 1e4, "cuda"))
+    q, k = _rand(batch, seq, heads, dim, seed=1), _rand(batch, seq, kv, dim, seed=2)
+    gq = _rand(batch, heads, seq, dim, seed=3).transpose(1, 2)  # as attention hands it back
+    gk = _rand(batch, seq, kv, dim, seed=4)
+    a, b = q.clone().requires_grad_(True), k.clone().requires_grad_(True)
+    for use in ("both", "q"):
+        a.grad = b.grad = None
+        qo, ko = C.rope(a, b, cos, sin)
+        torch.autograd.backward([qo, ko] if use == "both" else [qo], [gq, gk] if use == "both" else [gq])
+        for x, y, grad, g in ((q, qo, a.grad, gq), (k, ko, b.grad, gk)):
+            x64 = x.double().requires_grad_(True)
+            y64 = _apply_rope(x64.transpose(1, 2), cos.double(), sin.double()).transpose(1, 2)
+            y64.backward(g.double())
+            # the two products cancel: one rounding of the larger of them
+            bound = 1.01 * 2.0 ** -8 * y64.detach().abs() + 1e-6
+            assert ((y.detach().double() - y64.detach()).abs() <= bound).all()
+            if use == "q" and x is k:
+                assert grad is None or grad.abs().max() == 0
+            else:
+                assert ((grad.double() - x64.grad).abs() <= 1.01 * 2.0 ** -8 * x64.grad.abs() + 1e-6).all()
+
+
+def test_model_takes_the_torch_route_where_kernels_may_not_run():
+    """Autocast, function modes and second derivatives of the whole model still work, and
+    the two routes agree."""
+    model = build_llama(tiny_llama(), device="cuda", seed=1)
+    ids = torch.randint(0, 1024, (2, 33), device="cuda")
+
+    class Watch(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    C = _ext.load(required=True)
+    with torch.no_grad():
+        n0 = C.launch_count()
+        kernels = model(ids)
+        n1 = C.launch_count()
+        with Watch():
+            torch_route = model(ids)
+        assert n1 > n0 and C.launch_count() == n1
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert torch.allclose(model(ids).float(), torch_route.float(), rtol=0.1, atol=0.1)
+    assert (kernels.float() - torch_route.float()).norm() <= 2e-2 * torch_route.float().norm()
+    w = model.model.layers[0].mlp.gate_proj.weight
+    g, = torch.autograd.grad(model(ids).float().square().mean(), w, create_graph=False)
+    assert g.isfinite().all()
+    assert torch.func.jvp(lambda x: model.model.layers[0].mlp(x), (_rand(3, 256),), (_rand(3, 256),))[1].isfinite().all()
