@@ -1,9 +1,11 @@
 // Python bindings of the quantization kernels.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
 #include <optional>
 
+#include "qgemv.h"
 #include "quant.h"
 
 namespace py = pybind11;
@@ -107,6 +109,41 @@ void fake_quant(int64_t format, const Tensor& x, Tensor out, int64_t group, int6
                             (int)scale_dtype, ap, cur()), "fake_quant");
 }
 
+// x (..., cols) times the packed weight's transpose, for a few tokens; nullopt when the
+// kernel does not take the call (shape, dtype, layout or alignment).
+std::optional<Tensor> qgemv(int64_t format, const Tensor& packed, const Tensor& scales, const std::optional<Tensor>& global_scale,
+                            int64_t group, int64_t rows, int64_t cols, const Tensor& x, const std::optional<Tensor>& bias) {
+  if (x.dim() < 1 || x.size(-1) != cols || cols <= 0 || x.scalar_type() != at::kBFloat16) return std::nullopt;
+  const int64_t tokens = x.numel() / cols;
+  if (!oab::qgemv_supported((int)format, rows, cols, tokens, (int)group)) return std::nullopt;
+  const bool has_bias = bias.has_value() && bias->defined();
+  auto here = [&](const Tensor& t) { return t.device() == x.device() && t.is_contiguous(); };
+  if (!x.is_cuda() || !here(packed) || !here(scales)) return std::nullopt;
+  if (has_bias && (!here(*bias) || bias->scalar_type() != at::kBFloat16 || bias->dim() != 1 || bias->numel() != rows)) return std::nullopt;
+  // what the kernel reads has to be there, in the type that it expects
+  const int64_t n = rows * cols;
+  const float* gs = nullptr;
+  if (format == oab::kQInt8) {
+    if (packed.numel() != n || scales.numel() != rows || scales.scalar_type() != at::kBFloat16) return std::nullopt;
+  } else if (format == oab::kQNF4) {
+    if (packed.numel() * 2 != n || scales.numel() * group != n || scales.scalar_type() != at::kFloat) return std::nullopt;
+  } else {
+    if (packed.numel() * 2 != n || scales.numel() * 16 != n || scales.element_size() != 1) return std::nullopt;
+    if (!global_scale.has_value() || global_scale->device() != x.device() || global_scale->scalar_type() != at::kFloat) return std::nullopt;
+    gs = global_scale->data_ptr<float>();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  const Tensor xc = x.contiguous();
+  const uintptr_t pa = reinterpret_cast<uintptr_t>(packed.data_ptr());
+  if ((reinterpret_cast<uintptr_t>(xc.data_ptr()) & 31u) || (pa & (format == oab::kQInt8 ? 15u : 7u))) return std::nullopt;
+  auto shape = x.sizes().vec();
+  shape.back() = rows;
+  Tensor y = at::empty(shape, x.options());
+  ok(oab::launch_qgemv((int)format, packed.data_ptr(), scales.data_ptr(), gs, (int)group, xc.data_ptr(), tokens,
+                       has_bias ? bias->data_ptr() : nullptr, y.data_ptr(), rows, cols, cur()), "qgemv");
+  return y;
+}
+
 }  // namespace
 
 void bind_quant(py::module_& m) {
@@ -119,6 +156,8 @@ void bind_quant(py::module_& m) {
   m.def("int8_dequantize", &int8_dequantize);
   m.def("int4_quantize", &int4_quantize);
   m.def("int4_dequantize", &int4_dequantize);
+  m.def("qgemv", &qgemv);
+  m.attr("QGEMV_MAX_TOKENS") = oab::kQGemvMaxTokens;
   m.def("fake_quant", &fake_quant, py::arg("format"), py::arg("x"), py::arg("out"), py::arg("group"),
         py::arg("scale_dtype"), py::arg("amax") = py::none());
 }

@@ -28,6 +28,9 @@ import torch
 from torch import Tensor
 from torch.utils._python_dispatch import return_and_correct_aliasing
 
+from .. import _ext
+from ..ops.dispatch import use_kernels
+
 aten = torch.ops.aten
 
 
@@ -38,6 +41,9 @@ class _WeightOnlyLinear(torch.autograd.Function):
     def forward(ctx, x: Tensor, weight: "QWeightBase", bias: Optional[Tensor] = None):
         ctx.save_for_backward(x, weight)
         ctx.has_bias = bias is not None
+        y = _few_tokens(x, weight, bias)
+        if y is not None:
+            return y
         w = weight.dequantize(dtype=x.dtype)
         y = x @ w.T
         return y if bias is None else y + bias
@@ -51,6 +57,21 @@ class _WeightOnlyLinear(torch.autograd.Function):
         gw = g2.T @ x.reshape(-1, weight.shape[1])
         gb = g2.sum(0) if ctx.has_bias else None
         return gx, gw, gb
+
+
+def _few_tokens(x, weight, bias):
+    """``x @ dequant(W)^T (+ b)`` from the packed words (``csrc/qgemv.cu``), or None when the
+    kernel does not take the call.  Up to ``QGEMV_MAX_TOKENS`` tokens the packed bytes bound
+    the layer, and a dense copy of the weight costs several times their traffic."""
+    if not (weight.FEW_TOKEN_KERNEL and use_kernels(x) and (bias is None or use_kernels(bias))):
+        return None
+    rows, cols = weight.shape
+    C = _ext.load(required=True)
+    if x.numel() > C.QGEMV_MAX_TOKENS * cols:
+        return None
+    packed, scales = (getattr(weight, k) for k in weight.KERNEL_PAYLOAD)
+    return C.qgemv(weight.KERNEL_FORMAT, packed, scales, getattr(weight, "global_scale", None),
+                   weight.kernel_group(), rows, cols, x, bias)
 
 
 class QWeightBase(Tensor):
@@ -146,6 +167,9 @@ class QWeightBase(Tensor):
     #: names of the two payload tensors those kernels write: packed values, then scales.
     KERNEL_FORMAT = 0
     KERNEL_PAYLOAD: Tuple[str, str] = ("", "")
+
+    #: True when the few-token linear kernels read this format
+    FEW_TOKEN_KERNEL = False
 
     def kernel_group(self) -> int:
         """Columns per scale of the fused kernels (NF4 block size, int4 group size)."""

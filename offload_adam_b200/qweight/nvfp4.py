@@ -181,6 +181,7 @@ class NVFP4QWeight(QWeightBase):
     USES_TENSOR_AMAX = True
     KERNEL_FORMAT = 1
     KERNEL_PAYLOAD = ("weight_packed", "block_scale_fp8")
+    FEW_TOKEN_KERNEL = True
 
     def kernel_group(self):
         return NVFP4_BLOCKSIZE

@@ -1,0 +1,80 @@
+"""Linear layers on one to eight tokens straight from the packed weight, against fp64."""
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from offload_adam_b200 import _ext
+from offload_adam_b200.qweight import Int4QWeight, Int8QWeight, NF4QWeight, NVFP4QWeight
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(cls, rows, cols, tokens, bias, **kw):
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols + tokens)
+
+    def normal(*shape, std=1.0):
+        return (torch.randn(*shape, device="cuda", generator=gen) * std).to(torch.bfloat16)
+
+    w = torch.nn.Parameter(cls.from_float(normal(rows, cols, std=0.02), **kw), requires_grad=False)
+    return w, normal(tokens, cols), normal(rows) if bias else None
+
+
+def _check(w, x, b, y):
+    dense = w.data.dequantize(torch.float32).double()
+    want = x.double() @ dense.T + (0 if b is None else b.double())
+    # one rounding to bf16, plus fp32 rounding of a sum of cols products
+    slack = 2.0 ** -20 * (x.double().abs() @ dense.abs().T + 1e-30)
+    assert y.shape == (*x.shape[:-1], w.shape[0]) and y.dtype == torch.bfloat16
+    assert ((y.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + slack).all()
+
+
+# rows around the three launch shapes (1, 592 and 4736 rows) and their remainders; columns
+# around one warp step (512) and one CTA step (2048)
+@pytest.mark.parametrize("cls,kw", [(NVFP4QWeight, {}), (NF4QWeight, {}), (NF4QWeight, {"blocksize": 16}),
+                                    (NF4QWeight, {"blocksize": 512}), (Int8QWeight, {})])
+@pytest.mark.parametrize("rows,cols", [(1, 512), (5, 1024), (591, 2048), (593, 4608), (4741, 512), (4736, 2560)])
+@pytest.mark.parametrize("tokens", [1, 2, 3, 5, 8])
+def test_few_tokens(cls, kw, rows, cols, tokens):
+    w, x, b = _case(cls, rows, cols, tokens, bias=tokens % 2 == 0, **kw)
+    C = _ext.load(required=True)
+    with torch.no_grad():
+        n0 = C.launch_count()
+        y = F.linear(x, w, b)
+        assert C.launch_count() == n0 + 1  # no de-quantization
+    _check(w, x, b, y)
+
+
+@pytest.mark.parametrize("cls,cols", [(NVFP4QWeight, 16), (NF4QWeight, 64), (Int8QWeight, 48)])
+def test_narrow_weights(cls, cols):
+    w, x, b = _case(cls, 33, cols, 4, bias=True)
+    with torch.no_grad():
+        _check(w, x.view(2, 2, cols), b, F.linear(x.view(2, 2, cols), w, b))
+
+
+def test_other_calls_keep_the_dense_route():
+    """More tokens, other dtypes, ragged columns, formats without the kernel, non-contiguous
+    or misaligned activations: same result as before."""
+    for cls, cols, tokens in ((NF4QWeight, 256, 9), (Int8QWeight, 36, 2), (Int4QWeight, 256, 1)):
+        w, x, b = _case(cls, 40, cols, tokens, bias=False)
+        with torch.no_grad():
+            assert torch.equal(F.linear(x, w), x @ w.data.dequantize(torch.bfloat16).T)
+    w, x, b = _case(NF4QWeight, 40, 256, 2, bias=False)
+    with torch.no_grad():
+        assert torch.equal(F.linear(x.half(), w), x.half() @ w.data.dequantize(torch.float16).T)
+        _check(w, x, None, F.linear(x.T.contiguous().T, w))          # strided
+        shifted = torch.empty(513, device="cuda", dtype=torch.bfloat16)[1:].view(2, 256).copy_(x)
+        y = F.linear(shifted, w)                                     # not 32-byte aligned
+        assert torch.equal(y, x @ w.data.dequantize(torch.bfloat16).T)
+
+
+def test_gradients_of_a_few_tokens():
+    w, x, b = _case(NF4QWeight, 96, 256, 3, bias=True)
+    w.requires_grad_(True)
+    x.requires_grad_(True)
+    y = F.linear(x, w, b)
+    gy = torch.ones_like(y)
+    y.backward(gy)
+    dense = w.data.dequantize(torch.bfloat16)
+    assert torch.equal(x.grad, gy @ dense)
+    assert torch.equal(w.grad, gy.T @ x.detach())
