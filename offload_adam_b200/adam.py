@@ -16,7 +16,7 @@ import torch
 from torch.optim.optimizer import Optimizer
 
 from ._master import MasterLoadingMixin, is_quant
-from .ops.adam_step import STEP_FNS
+from .ops.adam_step import STEP_FNS, adam_step_many
 
 STATE_DTYPES = {
     "stochastic_rounding": {"exp_avg": torch.bfloat16, "exp_avg_sq": torch.bfloat16},
@@ -95,12 +95,13 @@ class Adam(MasterLoadingMixin, Optimizer):
             with torch.enable_grad():
                 loss = closure()
         for group in self.param_groups:
-            beta1, beta2 = group["betas"]
+            pending = {}  # step count -> CUDA parameters due, in one launch together
             for p in group["params"]:
                 grad = p.grad
                 if grad is None:
                     continue
                 if grad.is_sparse:
+                    self._step_pending(group, pending)
                     raise RuntimeError("Sparse gradient is not supported")
                 state = self.state[p]
                 self._init_state_if_empty(p, state)
@@ -110,20 +111,30 @@ class Adam(MasterLoadingMixin, Optimizer):
                     self._warn_lossy_master_once(state)
                 tensors = {k: state[k] for k in self.config["states"]}
                 tensors["grad"] = grad if grad.dtype == torch.bfloat16 else grad.to(torch.bfloat16)
-                kw = {}
-                if self.mode == "stochastic_rounding":
-                    kw["seed"] = self._rng.getrandbits(63)
+                seed = self._rng.getrandbits(63) if self.mode == "stochastic_rounding" else 0
                 # a quantized weight has no bf16 image to write: only the master moves,
                 # then copy_ re-quantizes the packed payload from it
-                self.step_fn(
-                    None if quant else p.data, tensors, group["lr"], group["weight_decay"], beta1,
-                    beta2, group["eps"], state["step"],
-                    decoupled_weight_decay=self.decoupled_weight_decay, **kw,
-                )
-                if quant:
-                    p.data.copy_(state["master_params"])
-                    p.grad = None
+                pending.setdefault(state["step"], []).append((p, quant, tensors, seed))
+            self._step_pending(group, pending)
         return loss
+
+    def _step_pending(self, group, pending):
+        beta1, beta2 = group["betas"]
+        for step, items in pending.items():
+            cuda = [it for it in items if it[2]["grad"].is_cuda]
+            if cuda:
+                adam_step_many(self.mode, [(None if quant else p.data, tensors, seed) for p, quant, tensors, seed in cuda],
+                               group["lr"], group["weight_decay"], beta1, beta2, group["eps"], step,
+                               self.decoupled_weight_decay)
+            for p, quant, tensors, seed in items:
+                if not tensors["grad"].is_cuda:
+                    self.step_fn(None if quant else p.data, tensors, group["lr"], group["weight_decay"], beta1, beta2,
+                                 group["eps"], step, decoupled_weight_decay=self.decoupled_weight_decay,
+                                 **({"seed": seed} if self.mode == "stochastic_rounding" else {}))
+                if quant:
+                    p.data.copy_(tensors["master_params"])
+                    p.grad = None
+        pending.clear()
 
     # ------------------------------------------------------------- checkpoint
     @torch.no_grad()

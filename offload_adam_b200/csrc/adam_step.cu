@@ -132,6 +132,105 @@ cudaError_t launch_adam_step(const AdamStepArgs& a, cudaStream_t stream) {
 }
 
 // ----------------------------------------------------------------------------
+// Many tensors, one launch: the optimizer whose state lives on the GPU.
+//
+// A launch per tensor leaves the chip idle twice: small tensors (a norm weight is a
+// fraction of one wave) cost a launch each, and every large one ends in a partly filled
+// wave.  Here a CTA takes `chunk` consecutive elements of one tensor, whichever tensor
+// that is, and all tensors share one tail.  Measured on a B200, a step of 20 tensors of a
+// tiny model: 220 -> 117 us (host bound); 62 M parameters in 11 tensors, fp31_master: 238 ->
+// 178 us; 1.27 G parameters in 12 tensors, fp32_master: 4008 -> 3769 us (6.7 TB/s).
+// ----------------------------------------------------------------------------
+namespace {
+struct ManyTable {
+  int count;
+  int64_t chunk;  // elements per CTA, a multiple of kThreads * kVec
+  ManyEntry e[kManyTensors];
+};
+
+template <int MODE, bool DECOUPLED>
+__global__ void __launch_bounds__(kThreads, 3)
+adam_step_many_kernel(const __grid_constant__ ManyTable table, AdamScalars s) {
+  int lo = 0, hi = table.count - 1;  // the last tensor whose first CTA is not after this one
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (table.e[mid].first_block <= blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const ManyEntry& e = table.e[lo];
+  const Ptrs t{(uint16_t*)e.p, (const uint16_t*)e.g, nullptr, (uint16_t*)e.m, (uint16_t*)e.v, e.extra, nullptr};
+  const Peers none{};
+  const int64_t begin = (int64_t)(blockIdx.x - e.first_block) * table.chunk;
+  const int64_t end = begin + table.chunk < e.n ? begin + table.chunk : e.n;
+  const uint64_t seed = e.seed;
+  int64_t scalar_begin = begin;
+  if (e.vector_ok) {
+    const int64_t vec_end = end / kVec;
+    scalar_begin = vec_end * kVec;
+    for (int64_t vec = begin / kVec + threadIdx.x; vec < vec_end; vec += kThreads) {
+      VecRegs<MODE> r;
+      load_vec<MODE, false, false>(r, t, none, vec);
+      compute_vec<MODE, DECOUPLED, false, false>(r, vec, 1.0f, s, seed, 0);
+      store_vec<MODE, false>(r, t, none, vec);
+    }
+  }
+  for (int64_t i = scalar_begin + threadIdx.x; i < end; i += kThreads)
+    scalar_element<MODE, DECOUPLED>(t, i, false, 1.0f, s, seed, 0);
+}
+
+template <int MODE>
+void launch_many(const ManyTable& t, unsigned grid, bool decoupled, const AdamScalars& s, cudaStream_t st) {
+  if (decoupled) adam_step_many_kernel<MODE, true><<<grid, kThreads, 0, st>>>(t, s);
+  else adam_step_many_kernel<MODE, false><<<grid, kThreads, 0, st>>>(t, s);
+}
+}  // namespace
+
+cudaError_t launch_adam_step_many(ManyEntry* entries, int count, int mode, bool decoupled, float lr, float wd,
+                                  float beta1_hat, float beta2_hat, float eps, cudaStream_t stream) {
+  AdamScalars s;
+  s.lr = lr; s.wd = wd; s.lr_wd = lr * wd;
+  s.one_m_b1h = 1.0f - beta1_hat; s.one_m_b2h = 1.0f - beta2_hat; s.eps = eps;
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
+  for (int at = 0; at < count; at += kManyTensors) {
+    ManyTable t;
+    t.count = 0;
+    int64_t total = 0;
+    for (int i = at; i < count && i < at + kManyTensors; ++i) {
+      const ManyEntry& e = entries[i];
+      if (e.g == nullptr || e.m == nullptr || e.v == nullptr) return cudaErrorInvalidValue;
+      if (mode != kModeFP32Master && e.p == nullptr) return cudaErrorInvalidValue;
+      if (mode != kModeSR && e.extra == nullptr) return cudaErrorInvalidValue;
+      if (e.n <= 0) continue;
+      total += e.n;
+      ManyEntry& o = t.e[t.count++];
+      o = e;
+      o.vector_ok = al(e.p) && al(e.g) && al(e.m) && al(e.v) && al(e.extra);
+    }
+    if (t.count == 0) continue;
+    // one vector per thread while that does not fill the chip several times over, four
+    // after that (a CTA's fixed cost is then a small part of its 10 us)
+    const int64_t unit = kThreads * kVec;
+    t.chunk = total >= unit * 4 * kNumSMs * 12 ? unit * 4 : unit;
+    int64_t blocks = 0;
+    for (int i = 0; i < t.count; ++i) {
+      t.e[i].first_block = (uint32_t)blocks;
+      blocks += (t.e[i].n + t.chunk - 1) / t.chunk;
+    }
+    if (blocks >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
+    count_launch();
+    switch (mode) {
+      case kModeSR: launch_many<kModeSR>(t, (unsigned)blocks, decoupled, s, stream); break;
+      case kModeFP32Master: launch_many<kModeFP32Master>(t, (unsigned)blocks, decoupled, s, stream); break;
+      case kModeFP31: launch_many<kModeFP31>(t, (unsigned)blocks, decoupled, s, stream); break;
+      case kModeCustom: launch_many<kModeCustom>(t, (unsigned)blocks, decoupled, s, stream); break;
+      default: return cudaErrorInvalidValue;
+    }
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
+}
+
+// ----------------------------------------------------------------------------
 // Multi-tensor variant: one launch updates every small (GPU-resident) tensor.
 // block_map[b] = {tensor index, chunk index}; each block handles kChunk elements.
 // (reference: the per-parameter loop of OffloadAdam._step_inplace,

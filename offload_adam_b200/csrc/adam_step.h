@@ -61,6 +61,25 @@ struct AdamStepArgs {
 // Enqueues one launch on `stream`.  Returns cudaGetLastError().
 cudaError_t launch_adam_step(const AdamStepArgs& a, cudaStream_t stream);
 
+// One tensor of launch_adam_step_many.
+struct ManyEntry {
+  void* p;
+  const void* g;
+  void* m;
+  void* v;
+  void* extra;
+  int64_t n;
+  uint64_t seed;
+  uint32_t first_block;  // filled in by the launch, as is vector_ok
+  uint32_t vector_ok;
+};
+// Steps `count` tensors that share mode and hyper-parameters, kManyTensors per launch; the
+// table travels as a kernel argument.  Each tensor gets the bits of its own
+// launch_adam_step (elem_offset 0, no clip, no peers).
+constexpr int kManyTensors = 120;
+cudaError_t launch_adam_step_many(ManyEntry* entries, int count, int mode, bool decoupled, float lr, float wd,
+                                  float beta1_hat, float beta2_hat, float eps, cudaStream_t stream);
+
 // Table-driven step over many small tensors in one launch.
 struct MultiTensorEntry {
   void* p;

@@ -132,6 +132,25 @@ void adam_step(int64_t mode, const OptT& p, const OptT& g, const OptT& g2, const
   cu_check(oab::launch_adam_step(a, pick_stream(stream)), "adam_step launch");
 }
 
+// The same step over many tensors with common hyper-parameters: lists of equal length, a
+// null parameter where only the master moves, no extra state for stochastic rounding.
+void adam_step_many(int64_t mode, const std::vector<OptT>& p, const std::vector<Tensor>& g, const std::vector<Tensor>& m,
+                    const std::vector<Tensor>& v, const std::vector<OptT>& extra, const std::vector<int64_t>& seeds,
+                    double lr, double wd, double b1h, double b2h, double eps, bool decoupled) {
+  const size_t k = g.size();
+  TORCH_CHECK(p.size() == k && m.size() == k && v.size() == k && extra.size() == k && seeds.size() == k,
+              "adam_step_many: lists of one length");
+  std::vector<oab::ManyEntry> e(k);
+  for (size_t i = 0; i < k; ++i) {
+    const auto a = make_args(mode, p[i], OptT(g[i]), OptT(), m[i], v[i], extra[i], lr, wd, b1h, b2h, eps, decoupled,
+                             OptT(), seeds[i], 0, OptT(), 0);
+    e[i] = {a.p, a.g, a.m, a.v, a.extra, a.n, a.seed, 0, 0};
+  }
+  cu_check(oab::launch_adam_step_many(e.data(), (int)k, (int)mode, decoupled, (float)lr, (float)wd, (float)b1h, (float)b2h,
+                                      (float)eps, pick_stream(0)),
+           "adam_step_many launch");
+}
+
 void grad_accumulate(const OptT& out, const Tensor& a, const OptT& b, const OptT& sumsq,
                      bool sumsq_accumulate, const OptT& scratch, int64_t max_ctas, int64_t stream) {
   TORCH_CHECK(a.scalar_type() == at::kBFloat16, "grad_accumulate: bf16 only");
@@ -455,6 +474,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("scratch") = py::none(), py::arg("max_ctas") = 0, py::arg("stream") = 0);
   m.def("clip_finalize", &clip_finalize, py::arg("slots"), py::arg("index"), py::arg("extra_sq"),
         py::arg("max_norm"), py::arg("coef_norm"), py::arg("total_sq"), py::arg("stream") = 0);
+  m.def("adam_step_many", &adam_step_many);
   m.def("multi_tensor_adam", &multi_tensor_adam);
   m.def("multi_tensor_chunk", &oab::multi_tensor_chunk);
   m.def("sumsq_scratch_bytes", []() { return (int64_t)oab::kSumsqScratchBytes; });
