@@ -26,18 +26,21 @@ cudaStream_t cur() { return at::cuda::getCurrentCUDAStream().stream(); }
 void ok(cudaError_t e, const char* what) { TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e)); }
 void dense(const Tensor& t, const char* n) { TORCH_CHECK(t.is_cuda() && t.is_contiguous(), n, " must be a contiguous CUDA tensor"); }
 
-void absmax(const Tensor& x, Tensor out) {
+// max |x| of disjoint parts of x; the largest is the tensor's
+Tensor absmax_partials(const Tensor& x) {
   dense(x, "x");
-  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kFloat && out.numel() >= 1, "out: CUDA fp32");
-  ok(oab::launch_absmax(x.data_ptr(), qdtype(x), x.numel(), out.data_ptr<float>(), cur()), "absmax");
+  Tensor out = at::empty({oab::absmax_partials(x.numel())}, x.options().dtype(at::kFloat));
+  ok(oab::launch_absmax_partials(x.data_ptr(), qdtype(x), x.numel(), out.data_ptr<float>(), cur()), "absmax_partials");
+  return out;
 }
 
 void nvfp4_quantize(const Tensor& x, const Tensor& amax, Tensor packed, Tensor scales, Tensor global_scale) {
   dense(x, "x"); dense(packed, "packed"); dense(scales, "scales");
   TORCH_CHECK(x.numel() % 16 == 0 && packed.numel() * 2 == x.numel() && scales.numel() * 16 == x.numel(), "nvfp4 shapes");
   TORCH_CHECK(packed.element_size() == 1 && scales.element_size() == 1, "nvfp4 payload dtypes");
+  TORCH_CHECK(amax.is_contiguous() && amax.numel() >= 1, "amax: one or more contiguous values");
   TORCH_CHECK(amax.is_cuda() && amax.scalar_type() == at::kFloat && global_scale.is_cuda() && global_scale.scalar_type() == at::kFloat, "scalars: CUDA fp32");
-  ok(oab::launch_nvfp4_quantize(x.data_ptr(), qdtype(x), x.numel(), amax.data_ptr<float>(),
+  ok(oab::launch_nvfp4_quantize(x.data_ptr(), qdtype(x), x.numel(), amax.data_ptr<float>(), (int)amax.numel(),
                                 (uint8_t*)packed.data_ptr(), (uint8_t*)scales.data_ptr(),
                                 global_scale.data_ptr<float>(), cur()), "nvfp4_quantize");
 }
@@ -101,12 +104,15 @@ void fake_quant(int64_t format, const Tensor& x, Tensor out, int64_t group, int6
   dense(x, "x"); dense(out, "out");
   TORCH_CHECK(x.dim() == 2 && out.sizes() == x.sizes() && out.scalar_type() == x.scalar_type(), "fake_quant: out like x (2-D)");
   const float* ap = nullptr;
+  int n_amax = 0;
   if (amax.has_value() && amax->defined()) {
-    TORCH_CHECK(amax->is_cuda() && amax->scalar_type() == at::kFloat, "amax: CUDA fp32");
+    TORCH_CHECK(amax->is_cuda() && amax->scalar_type() == at::kFloat && amax->is_contiguous() && amax->numel() >= 1,
+                "amax: contiguous CUDA fp32");
     ap = amax->data_ptr<float>();
+    n_amax = (int)amax->numel();
   }
   ok(oab::launch_fake_quant((int)format, x.data_ptr(), out.data_ptr(), qdtype(x), x.size(0), x.size(1), (int)group,
-                            (int)scale_dtype, ap, cur()), "fake_quant");
+                            (int)scale_dtype, ap, n_amax, cur()), "fake_quant");
 }
 
 // x (..., cols) times the packed weight's transpose, for a few tokens; nullopt when the
@@ -147,7 +153,7 @@ std::optional<Tensor> qgemv(int64_t format, const Tensor& packed, const Tensor& 
 }  // namespace
 
 void bind_quant(py::module_& m) {
-  m.def("absmax", &absmax);
+  m.def("absmax_partials", &absmax_partials);
   m.def("nvfp4_quantize", &nvfp4_quantize);
   m.def("nvfp4_dequantize", &nvfp4_dequantize);
   m.def("nf4_quantize", &nf4_quantize);

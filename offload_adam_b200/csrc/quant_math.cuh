@@ -20,12 +20,14 @@ constexpr float kEps = 1e-12f;
 
 // ------------------------------------------------------------------ element I/O
 template <typename T> struct Elem;
+// load16: data read once (evicted first); load16_keep: data that is read again soon
 template <> struct Elem<float> {
-  static __device__ __forceinline__ void load16(const float* p, float (&x)[16]) {
-    V8 a = ld32_stream(p), b = ld32_stream(p + 8);
+  static __device__ __forceinline__ void unpack(const V8& a, const V8& b, float (&x)[16]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) { x[i] = __uint_as_float(a.w[i]); x[8 + i] = __uint_as_float(b.w[i]); }
   }
+  static __device__ __forceinline__ void load16(const float* p, float (&x)[16]) { unpack(ld32_stream(p), ld32_stream(p + 8), x); }
+  static __device__ __forceinline__ void load16_keep(const float* p, float (&x)[16]) { unpack(ld32(p), ld32(p + 8), x); }
   static __device__ __forceinline__ void store16(float* p, const float (&x)[16]) {
     V8 a, b;
 #pragma unroll
@@ -36,11 +38,12 @@ template <> struct Elem<float> {
   static __device__ __forceinline__ float from_f32(float v) { return v; }
 };
 template <> struct Elem<__nv_bfloat16> {
-  static __device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&x)[16]) {
-    V8 a = ld32_stream(p);
+  static __device__ __forceinline__ void unpack(const V8& a, float (&x)[16]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) { x[2 * i] = __uint_as_float(a.w[i] << 16); x[2 * i + 1] = __uint_as_float(a.w[i] & 0xffff0000u); }
   }
+  static __device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&x)[16]) { unpack(ld32_stream(p), x); }
+  static __device__ __forceinline__ void load16_keep(const __nv_bfloat16* p, float (&x)[16]) { unpack(ld32(p), x); }
   static __device__ __forceinline__ void store16(__nv_bfloat16* p, const float (&x)[16]) {
     V8 a;
 #pragma unroll
@@ -51,15 +54,16 @@ template <> struct Elem<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 from_f32(float v) { return __float2bfloat16_rn(v); }
 };
 template <> struct Elem<__half> {
-  static __device__ __forceinline__ void load16(const __half* p, float (&x)[16]) {
-    V8 a = ld32_stream(p);
+  static __device__ __forceinline__ void unpack(const V8& a, float (&x)[16]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      __half2 h = *reinterpret_cast<__half2*>(&a.w[i]);
-      float2 f = __half22float2(h);
+      const __half2 h = *reinterpret_cast<const __half2*>(&a.w[i]);
+      const float2 f = __half22float2(h);
       x[2 * i] = f.x; x[2 * i + 1] = f.y;
     }
   }
+  static __device__ __forceinline__ void load16(const __half* p, float (&x)[16]) { unpack(ld32_stream(p), x); }
+  static __device__ __forceinline__ void load16_keep(const __half* p, float (&x)[16]) { unpack(ld32(p), x); }
   static __device__ __forceinline__ void store16(__half* p, const float (&x)[16]) {
     V8 a;
 #pragma unroll

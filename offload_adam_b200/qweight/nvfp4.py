@@ -120,8 +120,7 @@ def _quantize_nvfp4_cuda(tensor: Tensor, packed=None, scale=None, gscale=None, a
         scale = torch.empty((out_f, in_f // NVFP4_BLOCKSIZE), dtype=torch.float8_e4m3fn, device=dev)
         gscale = torch.empty((), dtype=torch.float32, device=dev)
     if amax is None:
-        amax = torch.zeros(1, dtype=torch.float32, device=dev)
-        C.absmax(src, amax)
+        amax = C.absmax_partials(src)
     C.nvfp4_quantize(src, amax, packed, scale, gscale)
     return packed, scale, gscale
 

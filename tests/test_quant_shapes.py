@@ -1,0 +1,51 @@
+"""Quantization kernels at the sizes where their launch rules change, bit for bit against
+the PyTorch restatements."""
+
+import pytest
+import torch
+
+from offload_adam_b200.qweight import Int8QWeight, NVFP4QWeight, fake_quantize
+from offload_adam_b200.qweight.int8 import _quantize_int8_cuda, quantize_int8_per_channel
+from offload_adam_b200.qweight.nvfp4 import _quantize_nvfp4_cuda, quantize_nvfp4_blockwise
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(rows, cols, dtype, shift=0):
+    gen = torch.Generator(device="cuda").manual_seed(rows * 131 + cols)
+    flat = torch.randn(rows * cols + shift, device="cuda", generator=gen).to(dtype)[shift:]
+    return flat.view(rows, cols)  # `shift` elements past a 512-byte boundary
+
+
+def _bits(t):
+    return t.cpu().contiguous().reshape(-1).view(torch.uint8)
+
+
+# quads of a warp end at 2048 columns, vectors of a CTA at 16384, quads of a CTA at 16384
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("cols", [4, 124, 1100, 2044, 2048, 2052, 4096, 16380, 16384, 16388])
+@pytest.mark.parametrize("rows", [1, 7, 9, 300])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_int8_rows(dtype, cols, rows, shift):
+    x = _rand(rows, cols, dtype, shift)
+    if rows > 1:
+        x[1] = 0
+    q, s = _quantize_int8_cuda(x, torch.bfloat16)
+    q_ref, s_ref = quantize_int8_per_channel(x.cpu(), scale_dtype=torch.bfloat16)
+    assert torch.equal(q.cpu(), q_ref) and torch.equal(s.cpu(), s_ref)
+    fake = fake_quantize(x, Int8QWeight)
+    assert torch.equal(_bits(fake), _bits(Int8QWeight(q, s).dequantize(dtype)))
+
+
+# one block; around a warp's 32 blocks; several CTAs; more than one sweep of the grid
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 16), (1, 496), (3, 176), (33, 512), (130, 4112), (2500, 4096)])
+def test_nvfp4_two_passes(dtype, rows, cols):
+    x = _rand(rows, cols, dtype)
+    x[-1, -1] = 40.0  # the maximum is in the last value
+    got = _quantize_nvfp4_cuda(x)
+    want = quantize_nvfp4_blockwise(x.cpu())
+    for a, b in zip(got, want):
+        assert torch.equal(_bits(a.reshape(b.shape)), _bits(b))
+    q = NVFP4QWeight(*got, cols, dtype)
+    assert torch.equal(_bits(fake_quantize(x, NVFP4QWeight)), _bits(q.dequantize(dtype)))
