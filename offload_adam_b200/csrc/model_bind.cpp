@@ -109,10 +109,97 @@ struct Rope : torch::autograd::Function<Rope> {
   }
 };
 
+// -------------------------------------------------------------------- RMSNorm
+bool norm_layout(const Tensor& t) {
+  return t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+}
+Tensor norm_operand(const Tensor& t) { return norm_layout(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
+
+// r defined: {x + r, norm(x + r) * w}; else {norm(x) * w}
+variable_list norm_forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+  check_bf16(x, "x");
+  check_bf16(w, "weight");
+  const int64_t cols = x.size(-1);
+  TORCH_CHECK(cols % 8 == 0 && cols <= oab::kNormMaxCols && w.dim() == 1 && w.size(0) == cols, "rms_norm: unsupported shape");
+  const bool add = r.defined();
+  if (add) {
+    check_bf16(r, "residual");
+    TORCH_CHECK(r.sizes() == x.sizes() && r.device() == x.device(), "rms_norm: residual like x");
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t rows = x.numel() / cols;
+  const Tensor xc = norm_operand(x), rc = add ? norm_operand(r) : r, wc = norm_operand(w);
+  Tensor out = at::empty(x.sizes(), x.options()), sum = add ? at::empty(x.sizes(), x.options()) : Tensor();
+  Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+  ok(oab::launch_rms_norm(xc.data_ptr(), add ? rc.data_ptr() : nullptr, wc.data_ptr(), add ? sum.data_ptr() : nullptr,
+                          out.data_ptr(), rstd.data_ptr<float>(), rows, (int)cols, (float)eps, cur()), "rms_norm");
+  ctx->set_materialize_grads(false);
+  ctx->saved_data["eps"] = eps;
+  ctx->save_for_backward({add ? sum : x, w, rstd});
+  if (add) return {sum, out};
+  return {out};
+}
+// {dx, dw} from the gradients of the sum (may be undefined) and of the norm
+variable_list norm_backward(AutogradContext* ctx, const Tensor& gsum, const Tensor& g, bool want_w) {
+  if (!g.defined()) return {gsum, Tensor()};
+  const auto saved = ctx->get_saved_variables();
+  const Tensor &x = saved[0], &w = saved[1], &rstd = saved[2];
+  Tensor dx, dw;
+  if (at::GradMode::is_enabled()) {  // a graph of the gradient is asked for
+    const Tensor x32 = x.to(at::kFloat);
+    const Tensor rs = at::rsqrt(x32.square().mean({-1}, true) + ctx->saved_data["eps"].toDouble());
+    const Tensor h = x32 * rs, gw = g.to(at::kFloat) * w.to(at::kFloat);
+    dx = (rs * (gw - h * (gw * h).mean({-1}, true))).to(x.scalar_type());
+    if (gsum.defined()) dx = dx + gsum;
+    dw = (g.to(at::kFloat) * h).reshape({-1, w.size(0)}).sum(0).to(w.scalar_type());
+    return {dx, dw};
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  const Tensor gc = norm_operand(g.to(at::kBFloat16)), xc = norm_operand(x), wc = norm_operand(w), rc = rstd.contiguous();
+  const Tensor sc = gsum.defined() ? norm_operand(gsum.to(at::kBFloat16)) : gsum;
+  dx = at::empty(x.sizes(), x.options());
+  Tensor partials;
+  if (want_w) {
+    dw = at::empty(w.sizes(), w.options());
+    partials = at::empty({(int64_t)oab::rms_norm_partials(rows, (int)cols) * cols}, rstd.options());
+  }
+  ok(oab::launch_rms_norm_grad(gc.data_ptr(), sc.defined() ? sc.data_ptr() : nullptr, xc.data_ptr(), wc.data_ptr(),
+                               rc.data_ptr<float>(), dx.data_ptr(), want_w ? dw.data_ptr() : nullptr,
+                               want_w ? partials.data_ptr<float>() : nullptr, rows, (int)cols, cur()), "rms_norm_grad");
+  return {dx, dw};
+}
+
+struct RmsNorm : torch::autograd::Function<RmsNorm> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, double eps) {
+    return norm_forward(ctx, x, Tensor(), w, eps)[0];
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto d = norm_backward(ctx, Tensor(), grads[0], ctx->needs_input_grad(1));
+    return {d[0], d[1], Tensor()};
+  }
+};
+
+struct AddRmsNorm : torch::autograd::Function<AddRmsNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+    return norm_forward(ctx, x, r, w, eps);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto d = norm_backward(ctx, grads[0], grads[1], ctx->needs_input_grad(2));
+    return {d[0], d[0], d[1], Tensor()};
+  }
+};
+
 }  // namespace
 
 void bind_model(py::module_& m) {
   m.def("swiglu", [](const Tensor& g, const Tensor& u) { return SwiGLU::apply(g, u); });
+  m.def("rms_norm", [](const Tensor& x, const Tensor& w, double eps) { return RmsNorm::apply(x, w, eps); });
+  m.def("add_rms_norm", [](const Tensor& x, const Tensor& r, const Tensor& w, double eps) {
+    auto out = AddRmsNorm::apply(x, r, w, eps);
+    return std::make_pair(out[0], out[1]);
+  });
+  m.attr("NORM_MAX_COLS") = oab::kNormMaxCols;
   m.def("rope", [](const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
     auto out = Rope::apply(q, k, cos, sin);
     return std::make_pair(out[0], out[1]);

@@ -134,6 +134,171 @@ __global__ void __launch_bounds__(kThreads) rope_kernel(RopeArgs a) {
   *reinterpret_cast<uint4*>(y + half) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
 }
 
+// -------------------------------------------------------------------- RMSNorm
+// LANES threads share a row (32: a warp, 256: a CTA) and hold it in registers, VPT vectors
+// of 8 values each, so that every operand is read once.  Measured on a B200 for 4096 rows of
+// 4096: 12 us forward, 23 us with the sum in front (5.9 TB/s; as two operations 30 us), 23 and
+// 28 us backward plus 7 us for the weight gradient (as three operations 65 us).
+__device__ __forceinline__ void unpack8(const uint4& r, float (&x)[8]) {
+  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { x[2 * i] = lo_f32(w[i]); x[2 * i + 1] = hi_f32(w[i]); }
+}
+__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
+  return make_uint4(f32x2_to_bf16x2_rne(x[0], x[1]), f32x2_to_bf16x2_rne(x[2], x[3]), f32x2_to_bf16x2_rne(x[4], x[5]),
+                    f32x2_to_bf16x2_rne(x[6], x[7]));
+}
+// Sum over the LANES threads of a row, in all of them.  `red`: kThreads / 32 floats, two
+// sets used in turn, so that one barrier per call is enough.
+template <int LANES>
+__device__ __forceinline__ float row_sum(float v, float* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (LANES == 32) return v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+#pragma unroll
+  for (int i = 1; i < kThreads / 32; ++i) v = __fadd_rn(v, red[i]);
+  return v;
+}
+
+template <int LANES, int VPT, bool ADD>
+__global__ void __launch_bounds__(kThreads)
+rms_norm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ r, const uint16_t* __restrict__ w,
+                uint16_t* __restrict__ sum, uint16_t* __restrict__ out, float* __restrict__ rstd, int64_t rows, int cols,
+                float eps) {
+  __shared__ float red[kThreads / 32];
+  const int lane = threadIdx.x % LANES, nvec = cols >> 3;
+  const int64_t row = (int64_t)blockIdx.x * (kThreads / LANES) + threadIdx.x / LANES;
+  if (row >= rows) return;  // whole warps (LANES == 32) or the whole CTA
+  const int64_t base = row * cols;
+  float e[VPT][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int v = lane + k * LANES;
+    if (v >= nvec) continue;
+    unpack8(*reinterpret_cast<const uint4*>(x + base + v * 8), e[k]);
+    if (ADD) {
+      float a[8];
+      unpack8(*reinterpret_cast<const uint4*>(r + base + v * 8), a);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = __fadd_rn(e[k][i], a[i]);
+      const uint4 packed = pack8(a);
+      *reinterpret_cast<uint4*>(sum + base + v * 8) = packed;
+      unpack8(packed, e[k]);  // the norm is of the rounded sum, which the residual stream keeps
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss = __fmaf_rn(e[k][i], e[k][i], ss);
+  }
+  ss = row_sum<LANES>(ss, red);
+  const float rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)cols), eps)));
+  if (lane == 0) rstd[row] = rs;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int v = lane + k * LANES;
+    if (v >= nvec) continue;
+    float wv[8];
+    unpack8(__ldg(reinterpret_cast<const uint4*>(w + v * 8)), wv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wv[i] = __fmul_rn(__fmul_rn(e[k][i], rs), wv[i]);
+    *reinterpret_cast<uint4*>(out + base + v * 8) = pack8(wv);
+  }
+}
+
+// Every group of LANES threads walks rows with stride `groups` and keeps its share of the
+// weight gradient in registers; one row of partial sums per group goes to memory.
+template <int LANES, int VPT, bool GSUM>
+__global__ void __launch_bounds__(kThreads)
+rms_norm_grad_kernel(const uint16_t* __restrict__ g, const uint16_t* __restrict__ gsum, const uint16_t* __restrict__ x,
+                     const uint16_t* __restrict__ w, const float* __restrict__ rstd, uint16_t* __restrict__ dx,
+                     float* __restrict__ partials, int64_t rows, int cols, int groups) {
+  __shared__ float red[2][kThreads / 32];
+  const int lane = threadIdx.x % LANES, nvec = cols >> 3;
+  const int group = blockIdx.x * (kThreads / LANES) + threadIdx.x / LANES;
+  if (group >= groups) return;  // whole warps or the whole CTA
+  float acc[VPT][8];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[k][i] = 0.f;
+  const float inv_cols = __fdiv_rn(1.0f, (float)cols);
+  int turn = 0;
+  for (int64_t row = group; row < rows; row += groups, turn ^= 1) {
+    const int64_t base = row * cols;
+    const float rs = rstd[row];
+    uint4 gp[VPT], xp[VPT], sp[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int v = lane + k * LANES;
+      if (v >= nvec) continue;
+      gp[k] = *reinterpret_cast<const uint4*>(g + base + v * 8);
+      xp[k] = *reinterpret_cast<const uint4*>(x + base + v * 8);
+      if (GSUM) sp[k] = *reinterpret_cast<const uint4*>(gsum + base + v * 8);
+    }
+    float c = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int v = lane + k * LANES;
+      if (v >= nvec) continue;
+      float gv[8], xv[8], wv[8];
+      unpack8(gp[k], gv);
+      unpack8(xp[k], xv);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(w + v * 8)), wv);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float h = __fmul_rn(xv[i], rs);
+        acc[k][i] = __fmaf_rn(gv[i], h, acc[k][i]);
+        c = __fmaf_rn(__fmul_rn(gv[i], wv[i]), h, c);
+      }
+    }
+    c = __fmul_rn(row_sum<LANES>(c, red[turn]), inv_cols);
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int v = lane + k * LANES;
+      if (v >= nvec) continue;
+      float gv[8], xv[8], wv[8], o[8];
+      unpack8(gp[k], gv);
+      unpack8(xp[k], xv);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(w + v * 8)), wv);
+      if (GSUM) unpack8(sp[k], o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float d = __fmul_rn(rs, __fmaf_rn(-c, __fmul_rn(xv[i], rs), __fmul_rn(gv[i], wv[i])));
+        o[i] = GSUM ? __fadd_rn(d, o[i]) : d;
+      }
+      *reinterpret_cast<uint4*>(dx + base + v * 8) = pack8(o);
+    }
+  }
+  if (partials == nullptr) return;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int v = lane + k * LANES;
+    if (v >= nvec) continue;
+    float4* p = reinterpret_cast<float4*>(partials + (int64_t)group * cols + v * 8);
+    p[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+    p[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
+  }
+}
+
+// dw[c] = sum over the groups, 32 columns per CTA: 8 threads a column, then their 8 sums.
+__global__ void __launch_bounds__(kThreads)
+column_sum_kernel(const float* __restrict__ partials, int groups, int cols, uint16_t* __restrict__ dw) {
+  __shared__ float red[8][33];
+  const int c = threadIdx.x & 31, part = threadIdx.x >> 5, col = blockIdx.x * 32 + c;
+  float s = 0.f;
+  if (col < cols)
+    for (int i = part; i < groups; i += 8) s = __fadd_rn(s, partials[(int64_t)i * cols + col]);
+  red[part][c] = s;
+  __syncthreads();
+  if (part == 0 && col < cols) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s = __fadd_rn(s, red[i][c]);
+    dw[col] = (uint16_t)f32_to_bf16_rne_bits(s);
+  }
+}
+
 bool aligned(const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; }
 bool rope_ok(const RopeTensor& t) {
   return t.heads == 0 || (t.in != nullptr && t.out != nullptr && aligned(t.in, 16) && aligned(t.out, 16) &&
@@ -177,6 +342,60 @@ cudaError_t launch_rope(const RopeTensor& q, const RopeTensor& k, const void* co
   count_launch();
   if (transposed) rope_kernel<true><<<(unsigned)grid, kThreads, 0, st>>>(a);
   else rope_kernel<false><<<(unsigned)grid, kThreads, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+// A warp holds up to 1024 columns (four vectors a thread), a CTA up to 16384 (eight).
+#define OAB_NORM_SHAPE(...)                                                      \
+  do {                                                                           \
+    if (cols <= 1024) { constexpr int LANES = 32, VPT = 4; __VA_ARGS__; }        \
+    else if (cols <= 4096) { constexpr int LANES = kThreads, VPT = 2; __VA_ARGS__; } \
+    else if (cols <= 8192) { constexpr int LANES = kThreads, VPT = 4; __VA_ARGS__; } \
+    else { constexpr int LANES = kThreads, VPT = 8; __VA_ARGS__; }               \
+  } while (0)
+
+cudaError_t launch_rms_norm(const void* x, const void* r, const void* w, void* sum, void* out, float* rstd,
+                            int64_t rows, int cols, float eps, cudaStream_t st) {
+  if (rows <= 0 || cols <= 0) return cudaSuccess;
+  if (cols % 8 != 0 || cols > kNormMaxCols || rows >= kMaxGrid || !aligned(x, 16) || !aligned(r, 16) || !aligned(w, 16) ||
+      !aligned(sum, 16) || !aligned(out, 16) || (r != nullptr && sum == nullptr))
+    return cudaErrorInvalidValue;
+  count_launch();
+  OAB_NORM_SHAPE(
+      const unsigned grid = (unsigned)((rows + kThreads / LANES - 1) / (kThreads / LANES));
+      if (r != nullptr)
+        rms_norm_kernel<LANES, VPT, true><<<grid, kThreads, 0, st>>>((const uint16_t*)x, (const uint16_t*)r, (const uint16_t*)w, (uint16_t*)sum, (uint16_t*)out, rstd, rows, cols, eps);
+      else
+        rms_norm_kernel<LANES, VPT, false><<<grid, kThreads, 0, st>>>((const uint16_t*)x, nullptr, (const uint16_t*)w, nullptr, (uint16_t*)out, rstd, rows, cols, eps));
+  return cudaGetLastError();
+}
+
+// Groups of threads that share the rows: three CTAs per SM when a CTA holds a row, two CTAs
+// of eight warps per SM when a warp does.
+int rms_norm_partials(int64_t rows, int cols) {
+  const int64_t most = cols <= 1024 ? (int64_t)kNumSMs * 16 : (int64_t)kNumSMs * 3;
+  return (int)(rows < most ? rows : most);
+}
+
+cudaError_t launch_rms_norm_grad(const void* g, const void* gsum, const void* x, const void* w, const float* rstd,
+                                 void* dx, void* dw, float* partials, int64_t rows, int cols, cudaStream_t st) {
+  if (rows <= 0 || cols <= 0) return cudaSuccess;
+  if (cols % 8 != 0 || cols > kNormMaxCols || !aligned(g, 16) || !aligned(gsum, 16) || !aligned(x, 16) || !aligned(w, 16) ||
+      !aligned(dx, 16) || !aligned(partials, 16) || (dw != nullptr && partials == nullptr))
+    return cudaErrorInvalidValue;
+  const int groups = rms_norm_partials(rows, cols);
+  float* part = dw != nullptr ? partials : nullptr;
+  count_launch();
+  OAB_NORM_SHAPE(
+      const unsigned grid = (unsigned)((groups + kThreads / LANES - 1) / (kThreads / LANES));
+      if (gsum != nullptr)
+        rms_norm_grad_kernel<LANES, VPT, true><<<grid, kThreads, 0, st>>>((const uint16_t*)g, (const uint16_t*)gsum, (const uint16_t*)x, (const uint16_t*)w, rstd, (uint16_t*)dx, part, rows, cols, groups);
+      else
+        rms_norm_grad_kernel<LANES, VPT, false><<<grid, kThreads, 0, st>>>((const uint16_t*)g, nullptr, (const uint16_t*)x, (const uint16_t*)w, rstd, (uint16_t*)dx, part, rows, cols, groups));
+  if (dw != nullptr) {
+    count_launch();
+    column_sum_kernel<<<(unsigned)((cols + 31) / 32), kThreads, 0, st>>>(partials, groups, cols, (uint16_t*)dw);
+  }
   return cudaGetLastError();
 }
 

@@ -26,4 +26,18 @@ struct RopeTensor {
 cudaError_t launch_rope(const RopeTensor& q, const RopeTensor& k, const void* cos, const void* sin, int64_t batch,
                         int64_t seq, int dim, bool transposed, cudaStream_t st);
 
+// RMSNorm of rows of `cols` bf16 values (cols % 8 == 0, cols <= kNormMaxCols, 16-byte aligned):
+// sum = bf16(x + r) when r is given (else the row is x itself and `sum` is not written),
+// out = bf16(row * rstd * w) with rstd[i] = 1 / sqrt(mean(row^2) + eps).
+constexpr int kNormMaxCols = 16384;
+cudaError_t launch_rms_norm(const void* x, const void* r, const void* w, void* sum, void* out, float* rstd,
+                            int64_t rows, int cols, float eps, cudaStream_t st);
+
+// Gradients: dx = bf16(rstd (g w - xhat mean(g w xhat)) + gsum), xhat = x rstd; gsum (the
+// gradient of `sum`) may be null.  dw = bf16(sum over rows of g xhat) through `partials`,
+// rms_norm_partials(rows, cols) * cols floats; dw may be null.  Fixed summation order.
+cudaError_t launch_rms_norm_grad(const void* g, const void* gsum, const void* x, const void* w, const float* rstd,
+                                 void* dx, void* dw, float* partials, int64_t rows, int cols, cudaStream_t st);
+int rms_norm_partials(int64_t rows, int cols);
+
 }  // namespace oab

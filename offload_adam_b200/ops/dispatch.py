@@ -17,12 +17,13 @@ _PLAIN = (torch.Tensor, nn.Parameter)
 
 def eager():
     """True in ordinary eager execution: no transform, mode or tracer is active."""
+    if torch.compiler.is_compiling():  # first: a tracer need not look at the rest
+        return False
     return (torch._C._functorch.peek_interpreter_stack() is None
             and forward_ad._current_level < 0
             and not torch._C._len_torch_dispatch_stack()
             and not torch._C._len_torch_function_stack()
             and not torch.is_autocast_enabled("cuda")
-            and not torch.compiler.is_compiling()
             and not torch.jit.is_tracing())
 
 

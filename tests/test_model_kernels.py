@@ -78,6 +78,62 @@ def test_rope(dim, batch, seq, heads, kv):
                 assert ((grad.double() - x64.grad).abs() <= 1.01 * 2.0 ** -8 * x64.grad.abs() + 1e-6).all()
 
 
+def _norm64(x, w, eps):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * w
+
+
+# a warp's row ends at 1024 columns, a CTA's with 2, 4 and 8 vectors a thread at 4096, 8192
+# and 16384; rows around the groups that share them in backward (444 CTAs, 2368 warps)
+@pytest.mark.parametrize("cols", [8, 256, 840, 1024, 1032, 4096, 4104, 8192, 16384])
+@pytest.mark.parametrize("rows", [1, 9, 445, 2371])
+@pytest.mark.parametrize("add", [False, True])
+def test_rms_norm(cols, rows, add):
+    C = _ext.load(required=True)
+    x, r, g, gs = (_rand(rows, cols, seed=s) for s in range(4))
+    w = (1 + 0.1 * _rand(cols, seed=9).float()).to(torch.bfloat16).requires_grad_(True)
+    a, b = x.clone().requires_grad_(True), r.clone().requires_grad_(True)
+    if add:
+        s, n = C.add_rms_norm(a, b, w, 1e-5)
+        assert torch.equal(s.detach(), x + r)
+        torch.autograd.backward([s, n], [gs, g])
+    else:
+        n = C.rms_norm(a, w, 1e-5)
+        n.backward(g)
+    y = (x + r if add else x).double().requires_grad_(True)
+    w64 = w.detach().double().requires_grad_(True)
+    n64 = _norm64(y, w64, 1e-5)
+    torch.autograd.backward([n64, y * 1.0] if add else [n64], [g.double(), gs.double()] if add else [g.double()])
+    _close(n.detach(), n64.detach())
+    # fp32 sums over a row and over the rows: relative to what is summed
+    assert ((a.grad.double() - y.grad).abs() <= 1.01 * 2.0 ** -8 * y.grad.abs() + 1e-5).all()
+    slack = 2.0 ** -20 * (g.double() * y.detach()).abs().sum(0)
+    assert ((w.grad.double() - w64.grad).abs() <= 1.01 * 2.0 ** -8 * w64.grad.abs() + slack).all()
+    assert not add or torch.equal(a.grad, b.grad)
+
+
+def test_rms_norm_of_which_one_output_is_used_and_second_derivative():
+    C = _ext.load(required=True)
+    x, r = _rand(5, 64, seed=1).requires_grad_(True), _rand(5, 64, seed=2).requires_grad_(True)
+    w = torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    s, n = C.add_rms_norm(x, r, w, 1e-5)
+    gx, = torch.autograd.grad(s, x, torch.ones_like(s), retain_graph=True)
+    assert torch.equal(gx, torch.ones_like(gx))
+    gx, = torch.autograd.grad(n, x, torch.ones_like(n), create_graph=True)
+    hx, = torch.autograd.grad(gx.float().square().sum(), x)
+    y = (x + r).detach().double().requires_grad_(True)
+    g64, = torch.autograd.grad(_norm64(y, w.double(), 1e-5).sum(), y, create_graph=True)
+    h64, = torch.autograd.grad(g64.square().sum(), y)
+    assert (hx.double() - h64).norm() <= 5e-2 * h64.norm()
+
+
+def test_hooks_on_a_norm_still_see_its_calls():
+    model = build_llama(tiny_llama(), device="cuda", seed=1)
+    ids = torch.randint(0, 1024, (1, 9), device="cuda")
+    plain, seen = model(ids), []
+    model.model.layers[0].post_attention_layernorm.register_forward_hook(lambda m, i, o: seen.append(o))
+    assert torch.equal(model(ids), plain) and len(seen) == 1 and seen[0].shape == (1, 9, 256)
+
+
 def test_model_takes_the_torch_route_where_kernels_may_not_run():
     """Autocast, function modes and second derivatives of the whole model still work, and
     the two routes agree."""
