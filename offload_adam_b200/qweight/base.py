@@ -41,9 +41,6 @@ class _WeightOnlyLinear(torch.autograd.Function):
     def forward(ctx, x: Tensor, weight: "QWeightBase", bias: Optional[Tensor] = None):
         ctx.save_for_backward(x, weight)
         ctx.has_bias = bias is not None
-        y = _few_tokens(x, weight, bias)
-        if y is not None:
-            return y
         w = weight.dequantize(dtype=x.dtype)
         y = x @ w.T
         return y if bias is None else y + bias
@@ -59,19 +56,19 @@ class _WeightOnlyLinear(torch.autograd.Function):
         return gx, gw, gb
 
 
-def _few_tokens(x, weight, bias):
-    """``x @ dequant(W)^T (+ b)`` from the packed words (``csrc/qgemv.cu``), or None when the
-    kernel does not take the call.  Up to ``QGEMV_MAX_TOKENS`` tokens the packed bytes bound
-    the layer, and a dense copy of the weight costs several times their traffic."""
-    if not (weight.FEW_TOKEN_KERNEL and use_kernels(x) and (bias is None or use_kernels(bias))):
-        return None
-    rows, cols = weight.shape
-    C = _ext.load(required=True)
-    if x.numel() > C.QGEMV_MAX_TOKENS * cols:
-        return None
-    packed, scales = (getattr(weight, k) for k in weight.KERNEL_PAYLOAD)
-    return C.qgemv(weight.KERNEL_FORMAT, packed, scales, getattr(weight, "global_scale", None),
-                   weight.kernel_group(), rows, cols, x, bias)
+def _linear(input, weight, bias=None):
+    """``F.linear`` on a packed weight.  bf16 activations on CUDA take a C++ autograd node
+    (``csrc/quant_bind.cpp`` ``QLinear``); up to ``QGEMV_MAX_TOKENS`` tokens it multiplies
+    with the packed words directly (``csrc/qgemv.cu``).  Everything else takes the Python
+    node above."""
+    if (isinstance(weight, QWeightBase) and weight.KERNEL_FORMAT and use_kernels(input)
+            and (bias is None or use_kernels(bias))):
+        packed, scales = (getattr(weight, k) for k in weight.KERNEL_PAYLOAD)
+        y = _ext.load(required=True).qlinear(input, weight, bias, weight.KERNEL_FORMAT, weight.kernel_group(),
+                                             packed, scales, getattr(weight, "global_scale", None))
+        if y is not None:
+            return y
+    return _WeightOnlyLinear.apply(input, weight, bias)
 
 
 class QWeightBase(Tensor):
@@ -168,9 +165,6 @@ class QWeightBase(Tensor):
     KERNEL_FORMAT = 0
     KERNEL_PAYLOAD: Tuple[str, str] = ("", "")
 
-    #: True when the few-token linear kernels read this format
-    FEW_TOKEN_KERNEL = False
-
     def kernel_group(self) -> int:
         """Columns per scale of the fused kernels (NF4 block size, int4 group size)."""
         return 0
@@ -242,8 +236,8 @@ def _install_common_handlers(cls):
     """Handlers every format shares; a subclass may override any of them."""
 
     @cls.implements_torch_function(torch.nn.functional.linear)
-    def _linear(func, types, args, kwargs):
-        return _WeightOnlyLinear.apply(*args, **kwargs)
+    def _linear_handler(func, types, args, kwargs):
+        return _linear(*args, **kwargs)
 
     @cls.implements([aten.detach.default, aten.clone.default])
     def _detach_clone(func, types, args, kwargs):

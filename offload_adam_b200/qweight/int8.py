@@ -100,7 +100,6 @@ class Int8QWeight(QWeightBase):
 
     KERNEL_FORMAT = 4
     KERNEL_PAYLOAD = ("weight", "scales")
-    FEW_TOKEN_KERNEL = True
 
     def kernel_scale_dtype(self):
         return self.scales.dtype

@@ -145,7 +145,6 @@ class NF4QWeight(QWeightBase):
 
     KERNEL_FORMAT = 2
     KERNEL_PAYLOAD = ("weight_packed", "absmax")
-    FEW_TOKEN_KERNEL = True
 
     def kernel_group(self):
         return self.blocksize

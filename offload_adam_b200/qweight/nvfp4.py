@@ -15,6 +15,8 @@ restatements (CPU path and test oracle); on CUDA the sm_100a kernels in
 
 from __future__ import annotations
 
+import functools
+
 from typing import Tuple
 
 import torch
@@ -98,18 +100,17 @@ def dequantize_nvfp4_blockwise(packed, block_scale_fp8, global_scale, in_f, dtyp
     return (vals * eff).reshape(out_f, in_f).to(dtype)
 
 
-def _supports_native_fp4() -> bool:
-    """True when the CUDA kernels (hardware E2M1 converts, sm_100a) can run."""
-    if not torch.cuda.is_available():
-        return False
+@functools.lru_cache(maxsize=None)
+def _supports_native_fp4(device: torch.device) -> bool:
+    """True when the CUDA kernels (hardware E2M1 converts, sm_100a) can run on ``device``."""
     try:
-        return torch.cuda.get_device_capability()[0] >= 10
+        return torch.cuda.get_device_capability(device)[0] >= 10
     except Exception:
         return False
 
 
 def _quantize_nvfp4_cuda(tensor: Tensor, packed=None, scale=None, gscale=None, amax=None):
-    """Kernel path: amax pre-pass (skipped when ``amax`` is supplied, e.g. by the
+    """Kernel path: a pass for max|x| (skipped when ``amax`` is supplied, e.g. by the
     fused optimizer step) + one quantize pass writing straight into the payload."""
     C = _ext.load(required=True)
     out_f, in_f = tensor.shape
@@ -119,8 +120,6 @@ def _quantize_nvfp4_cuda(tensor: Tensor, packed=None, scale=None, gscale=None, a
         packed = torch.empty((out_f, in_f // 2), dtype=torch.uint8, device=dev)
         scale = torch.empty((out_f, in_f // NVFP4_BLOCKSIZE), dtype=torch.float8_e4m3fn, device=dev)
         gscale = torch.empty((), dtype=torch.float32, device=dev)
-    if amax is None:
-        amax = C.absmax_partials(src)
     C.nvfp4_quantize(src, amax, packed, scale, gscale)
     return packed, scale, gscale
 
@@ -171,7 +170,7 @@ class NVFP4QWeight(QWeightBase):
 
     def dequantize(self, dtype=None) -> Tensor:
         dtype = dtype or self.outer_dtype
-        if self.weight_packed.is_cuda and dtype in _CUDA_DTYPES and _supports_native_fp4():
+        if self.weight_packed.is_cuda and dtype in _CUDA_DTYPES and _supports_native_fp4(self.weight_packed.device):
             return _dequant_nvfp4_cuda(self.weight_packed, self.block_scale_fp8, self.global_scale,
                                        self.in_f, dtype)
         return dequantize_nvfp4_blockwise(self.weight_packed, self.block_scale_fp8, self.global_scale,
@@ -180,7 +179,6 @@ class NVFP4QWeight(QWeightBase):
     USES_TENSOR_AMAX = True
     KERNEL_FORMAT = 1
     KERNEL_PAYLOAD = ("weight_packed", "block_scale_fp8")
-    FEW_TOKEN_KERNEL = True
 
     def kernel_group(self):
         return NVFP4_BLOCKSIZE
@@ -189,7 +187,7 @@ class NVFP4QWeight(QWeightBase):
         return [self.weight_packed[lo:hi], self.block_scale_fp8[lo:hi], self.global_scale]
 
     def _quantize_into(self, src: Tensor, amax=None) -> None:
-        if self.weight_packed.is_cuda and src.is_cuda and src.dtype in _CUDA_DTYPES and _supports_native_fp4():
+        if self.weight_packed.is_cuda and src.is_cuda and src.dtype in _CUDA_DTYPES and _supports_native_fp4(self.weight_packed.device):
             _quantize_nvfp4_cuda(src, self.weight_packed, self.block_scale_fp8, self.global_scale, amax=amax)
             return
         packed, scale, gs = quantize_nvfp4_blockwise(src.to(self.weight_packed.device), amax=amax)

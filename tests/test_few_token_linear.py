@@ -78,3 +78,50 @@ def test_gradients_of_a_few_tokens():
     dense = w.data.dequantize(torch.bfloat16)
     assert torch.equal(x.grad, gy @ dense)
     assert torch.equal(w.grad, gy.T @ x.detach())
+
+
+@pytest.mark.parametrize("cls,kw", [(NVFP4QWeight, {}), (NF4QWeight, {}), (Int4QWeight, {"group_size": 64}), (Int8QWeight, {})])
+@pytest.mark.parametrize("shape", [(37,), (3, 11)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_autograd_node_matches_the_general_one(cls, kw, shape, bias):
+    """More tokens than the few-token kernel takes: the C++ node against the Python node."""
+    from offload_adam_b200.qweight.base import _WeightOnlyLinear
+
+    rows, cols = 96, 256
+    n = torch.Size(shape).numel()
+    w, x, b = _case(cls, rows, cols, n, bias, **kw)
+    x, gy = x.view(*shape, cols), _case(cls, rows, rows * 4, n, False)[1][:, :rows].reshape(*shape, rows)
+    out = []
+    for fn in (F.linear, _WeightOnlyLinear.apply):
+        wi = torch.nn.Parameter(w.data)
+        xi = x.clone().requires_grad_(True)
+        bi = torch.nn.Parameter(b.clone()) if bias else None
+        y = fn(xi, wi, bi)
+        y.backward(gy)
+        out.append([y.detach(), xi.grad, wi.grad] + ([bi.grad] if bias else []))
+    for i, (a, c) in enumerate(zip(*out)):
+        if i == 0 and bias:  # the sum with the bias rounds once, there twice
+            assert ((a.double() - c.double()).abs() <= 2.0 ** -7 * c.double().abs() + 2.0 ** -7).all()
+        else:
+            assert torch.equal(a, c)
+
+
+def test_autograd_node_with_frozen_inputs_and_second_derivative():
+    w, x, _ = _case(NF4QWeight, 64, 128, 20, False)
+    frozen = torch.nn.Parameter(w.data, requires_grad=False)
+    x.requires_grad_(True)
+    y = F.linear(x, frozen)
+    gx, = torch.autograd.grad(y.float().square().sum(), x, create_graph=True)
+    hx, = torch.autograd.grad(gx.float().sum(), x)
+    assert frozen.grad is None and hx.isfinite().all() and hx.abs().max() > 0
+    trained = torch.nn.Parameter(w.data)
+    F.linear(x.detach(), trained).sum().backward()  # only the weight needs a gradient
+    assert trained.grad.shape == (64, 128)
+    with torch.no_grad():
+        assert not F.linear(x, trained).requires_grad
+    mixed = torch.autograd.graph.save_on_cpu()
+    with mixed:
+        z = F.linear(x, trained)
+    g1, = torch.autograd.grad(z.sum(), x)
+    g2, = torch.autograd.grad(F.linear(x, trained).sum(), x)
+    assert torch.equal(g1, g2)
