@@ -1,6 +1,6 @@
 // y = x W^T (+ bias) for a few tokens and a packed weight, without a dense copy of it.
 //
-// A linear layer on one to eight tokens reads every weight once and does two to sixteen
+// A linear layer on one to four tokens reads every weight once and does two to eight
 // operations with it: the packed bytes are what it cannot do without.  De-quantizing to a
 // dense bf16 copy first writes and re-reads four (4-bit formats) or two (int8) times those
 // bytes.  Here the weights are decoded to fp32 in registers, multiplied with the bf16
@@ -9,7 +9,10 @@
 //
 // Row-major formats (NVFP4, NF4, int8): a lane owns 16 consecutive columns of R rows per
 // step, a warp 512 columns; the next step's words are loaded before the current ones are
-// used.  The R rows share the unpacked activations.
+// used.  The R rows share the unpacked activations.  One token through 14336 x 4096 NF4: 18 us
+// (1.8 TB/s of packed bytes), with a dense copy 46 us.  What bounds it is not the bytes but
+// the decoding: the look-ups of 58.7 M indices keep the shared-memory pipe busy for 6.5 us and
+// the issue slots 63 % of the time.
 #include "qgemv.h"
 #include "quant.h"
 #include "quant_math.cuh"
@@ -19,8 +22,7 @@ namespace {
 
 using namespace qm;
 
-constexpr int kThreads = 128;
-constexpr int kWarps = kThreads / 32;
+constexpr int kSplitWarps = 4;  // warps of a CTA that split a row
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   return ((uint64_t)__float_as_uint(hi) << 32) | __float_as_uint(lo);
@@ -104,18 +106,20 @@ __device__ __forceinline__ float scale_of(const Raw<FMT>& r) {
   return FMT == kQInt8 ? 1.0f : r.scale;
 }
 
-// SPLIT: the warps of a CTA share its R rows and split the columns; otherwise every warp
-// has R rows of its own.
+// SPLIT: the four warps of a CTA share its R rows and split the columns.  Otherwise a CTA is
+// one warp with R rows of its own: the rows of a layer rarely fill whole waves of larger
+// CTAs (14336 rows in CTAs of 16 are 896 of them where 888 fit at a time).
 template <int FMT, int R, int M, bool SPLIT>
-__global__ void __launch_bounds__(kThreads, M >= 4 ? 3 : (M == 2 ? 5 : 6)) qgemv_kernel(Args a) {
+__global__ void __launch_bounds__(SPLIT ? 32 * kSplitWarps : 32, (M == 4 ? 3 : (M == 2 ? 5 : 6)) * (SPLIT ? 1 : 4)) qgemv_kernel(Args a) {
+  constexpr int kWarps = SPLIT ? kSplitWarps : 1, kThreads = 32 * kWarps;
   __shared__ float lut[16];
   __shared__ float part[kWarps][R * M];
   if (FMT == kQNF4) {
     if (threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
-    __syncthreads();
+    if (SPLIT) __syncthreads(); else __syncwarp();
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row0 = SPLIT ? (int64_t)blockIdx.x * R : ((int64_t)blockIdx.x * kWarps + warp) * R;
+  const int64_t row0 = (int64_t)blockIdx.x * R;
   const int first = SPLIT ? threadIdx.x * 16 : lane * 16;
   const int step = SPLIT ? kThreads * 16 : 512;
   float acc[R][M];
@@ -171,8 +175,8 @@ __global__ void __launch_bounds__(kThreads, M >= 4 ? 3 : (M == 2 ? 5 : 6)) qgemv
       }
 #pragma unroll
       for (int t = 0; t < M; ++t) {
-        if (t >= a.tokens) break;
-        const V8 xv = ld32(a.x + (int64_t)t * a.cols + c);
+        // a missing fourth token repeats the last one: no branch between the loads
+        const V8 xv = ld32(a.x + (int64_t)(t < a.tokens ? t : a.tokens - 1) * a.cols + c);
         uint64_t p[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) p[r] = 0;
@@ -219,15 +223,104 @@ __global__ void __launch_bounds__(kThreads, M >= 4 ? 3 : (M == 2 ? 5 : 6)) qgemv
   }
 }
 
+// int4 (GPTQ layout): the words of one input position lie along the output rows, so a lane
+// owns a row, a warp reads 128 consecutive bytes per word, and the warps of a CTA split the
+// columns in units of 128 (16 words a lane, the next unit's loaded before the current one is
+// used).  The activations of a word are the same for all lanes: one broadcast load.
+template <int WORDS /* per quantization group */, int M, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) qgemv_int4_kernel(Args a) {
+  __shared__ float part[WARPS][M][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row0 = (int64_t)blockIdx.x * 32;
+  const int64_t row = row0 + lane < a.rows ? row0 + lane : a.rows - 1;
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a.w) + row;
+  const uint16_t* sc = reinterpret_cast<const uint16_t*>(a.scales) + row;
+  const int units = a.cols >> 7;
+  constexpr int kGroups = 16 / WORDS;
+  float acc[M];
+#pragma unroll
+  for (int t = 0; t < M; ++t) acc[t] = 0.f;
+  uint32_t nxt[16];
+  uint16_t nxs[kGroups];
+  auto load = [&](int u) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) nxt[k] = __ldcs(w + ((int64_t)u * 16 + k) * a.rows);
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) nxs[g] = __ldg(sc + ((int64_t)u * kGroups + g) * a.rows);
+  };
+  if (warp < units) load(warp);
+  for (int u = warp; u < units; u += WARPS) {
+    uint32_t cur[16];
+    float s[kGroups];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) cur[k] = nxt[k];
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) s[g] = bf16_bits_to_f32(nxs[g]);
+    if (u + WARPS < units) load(u + WARPS);
+    const uint16_t* x = a.x + u * 128;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+      uint64_t p[M];
+#pragma unroll
+      for (int t = 0; t < M; ++t) p[t] = 0;
+#pragma unroll
+      for (int k = 0; k < WORDS; ++k) {
+        const uint32_t v = cur[g * WORDS + k];
+        uint64_t q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          q[i] = pack2(small_int_to_f32((v >> (8 * i)) & 0xfu, 8388616.0f), small_int_to_f32((v >> (8 * i + 4)) & 0xfu, 8388616.0f));
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+          const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + (int64_t)t * a.cols + (g * WORDS + k) * 8));
+          p[t] = fma2(q[0], unpack_pair(xv.x), p[t]);
+          p[t] = fma2(q[1], unpack_pair(xv.y), p[t]);
+          p[t] = fma2(q[2], unpack_pair(xv.z), p[t]);
+          p[t] = fma2(q[3], unpack_pair(xv.w), p[t]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < M; ++t) acc[t] = __fmaf_rn(sum2(p[t]), s[g], acc[t]);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < M; ++t) part[warp][t][lane] = acc[t];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 32 * M; i += 32 * WARPS) {
+    const int t = i >> 5, l = i & 31;
+    if (t >= a.tokens || row0 + l >= a.rows) continue;
+    float v = part[0][t][l];
+#pragma unroll
+    for (int k = 1; k < WARPS; ++k) v = __fadd_rn(v, part[k][t][l]);
+    if (a.bias != nullptr) v = __fadd_rn(v, bf16_bits_to_f32(a.bias[row0 + l]));
+    a.y[(int64_t)t * a.rows + row0 + l] = (uint16_t)f32_to_bf16_rne_bits(v);
+  }
+}
+
+template <int WORDS, int M>
+cudaError_t launch_int4(const Args& a, cudaStream_t st) {
+  // fewer rows than a CTA of 32 per SM: more warps split the columns
+  const unsigned grid = (unsigned)((a.rows + 31) / 32);
+  if (a.rows >= int64_t(kNumSMs) * 32) qgemv_int4_kernel<WORDS, M, 8><<<grid, 256, 0, st>>>(a);
+  else qgemv_int4_kernel<WORDS, M, 16><<<grid, 512, 0, st>>>(a);
+  return cudaGetLastError();
+}
+template <int M>
+cudaError_t launch_int4_group(const Args& a, int group, cudaStream_t st) {
+  if (group == 32) return launch_int4<4, M>(a, st);
+  if (group == 64) return launch_int4<8, M>(a, st);
+  return launch_int4<16, M>(a, st);
+}
+
 template <int FMT, int M>
 cudaError_t launch_rows(const Args& a, cudaStream_t st) {
-  // Four rows per warp share the activations as long as that still gives every SM two CTAs;
-  // fewer rows: the warps of a CTA split the columns, so that a row's reads are in flight
-  // together; very few rows: one row per CTA.
+  // Four rows per warp share the activations as long as that still gives every SM eight
+  // warps; fewer rows: the warps of a CTA split the columns, so that a row's reads are in
+  // flight together; very few rows: one row per CTA.
   auto ctas = [&](int64_t per) { return (unsigned)((a.rows + per - 1) / per); };
-  if (a.rows >= int64_t(kNumSMs) * 2 * 4 * kWarps) qgemv_kernel<FMT, 4, M, false><<<ctas(4 * kWarps), kThreads, 0, st>>>(a);
-  else if (a.rows >= int64_t(kNumSMs) * 4) qgemv_kernel<FMT, 4, M, true><<<ctas(4), kThreads, 0, st>>>(a);
-  else qgemv_kernel<FMT, 1, M, true><<<ctas(1), kThreads, 0, st>>>(a);
+  if (a.rows >= int64_t(kNumSMs) * 32) qgemv_kernel<FMT, 4, M, false><<<ctas(4), 32, 0, st>>>(a);
+  else if (a.rows >= int64_t(kNumSMs) * 4) qgemv_kernel<FMT, 4, M, true><<<ctas(4), 32 * kSplitWarps, 0, st>>>(a);
+  else qgemv_kernel<FMT, 1, M, true><<<ctas(1), 32 * kSplitWarps, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -235,8 +328,7 @@ template <int FMT>
 cudaError_t launch_tokens(const Args& a, cudaStream_t st) {
   if (a.tokens == 1) return launch_rows<FMT, 1>(a, st);
   if (a.tokens == 2) return launch_rows<FMT, 2>(a, st);
-  if (a.tokens <= 4) return launch_rows<FMT, 4>(a, st);
-  return launch_rows<FMT, 8>(a, st);
+  return launch_rows<FMT, 4>(a, st);
 }
 
 }  // namespace
@@ -244,6 +336,7 @@ cudaError_t launch_tokens(const Args& a, cudaStream_t st) {
 bool qgemv_supported(int format, int64_t rows, int64_t cols, int64_t tokens, int group) {
   if (rows <= 0 || rows >= (int64_t(1) << 31) || cols <= 0 || cols % 16 != 0 || cols >= (int64_t(1) << 30)) return false;
   if (tokens < 1 || tokens > kQGemvMaxTokens) return false;
+  if (format == kQInt4) return tokens <= 2 && rows >= 1024 && cols % 128 == 0 && (group == 32 || group == 64 || group == 128);
   if (format == kQNF4) return group >= 16 && group <= 512 && (group & (group - 1)) == 0 && cols % group == 0;
   return format == kQNVFP4 || format == kQInt8;
 }
@@ -252,13 +345,15 @@ cudaError_t launch_qgemv(int format, const void* packed, const void* scales, con
                          const void* x, int64_t tokens, const void* bias, void* y, int64_t rows, int64_t cols,
                          cudaStream_t st) {
   if (!qgemv_supported(format, rows, cols, tokens, group)) return cudaErrorInvalidValue;
-  if ((reinterpret_cast<uintptr_t>(x) & 31u) || (reinterpret_cast<uintptr_t>(packed) & (format == kQInt8 ? 15u : 7u)))
+  if ((reinterpret_cast<uintptr_t>(x) & 31u) || (reinterpret_cast<uintptr_t>(packed) & (qgemv_packed_align(format) - 1)))
     return cudaErrorInvalidValue;
   Args a{(const uint8_t*)packed, scales, global_scale, (const uint16_t*)x, (const uint16_t*)bias, (uint16_t*)y,
          rows, (int)cols, (int)tokens, 0};
   while (format == kQNF4 && (1 << a.block_shift) < group) ++a.block_shift;
   count_launch();
   switch (format) {
+    case kQInt4:
+      return a.tokens == 1 ? launch_int4_group<1>(a, group, st) : launch_int4_group<2>(a, group, st);
     case kQNVFP4: return launch_tokens<kQNVFP4>(a, st);
     case kQNF4: return launch_tokens<kQNF4>(a, st);
     default: return launch_tokens<kQInt8>(a, st);
