@@ -190,6 +190,32 @@ struct AddRmsNorm : torch::autograd::Function<AddRmsNorm> {
   }
 };
 
+// ------------------------------------------------------------------ embedding
+struct Embedding : torch::autograd::Function<Embedding> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& weight, const Tensor& ids) {
+    check_bf16(weight, "embedding table");
+    TORCH_CHECK(weight.dim() == 2 && weight.size(1) % 8 == 0 && ids.scalar_type() == at::kLong && ids.device() == weight.device() &&
+                    ids.numel() <= oab::kEmbedMaxTokens, "embedding: unsupported call");
+    ctx->save_for_backward({ids});
+    ctx->saved_data["vocab"] = weight.size(0);
+    return at::embedding(weight, ids);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor ids = ctx->get_saved_variables()[0], &g = grads[0];
+    const int64_t vocab = ctx->saved_data["vocab"].toInt();
+    if (!g.defined()) return {Tensor(), Tensor()};
+    if (at::GradMode::is_enabled()) return {at::embedding_dense_backward(g, ids, vocab, -1, false), Tensor()};
+    c10::cuda::CUDAGuard guard(g.device());
+    const int64_t cols = g.size(-1), n = ids.numel();
+    const Tensor gc = norm_operand(g.to(at::kBFloat16)), ic = ids.contiguous();
+    Tensor dw = at::empty({vocab, cols}, gc.options());
+    Tensor work = at::empty({oab::embed_work_ints(n, vocab)}, gc.options().dtype(at::kInt));
+    ok(oab::launch_embed_grad(gc.data_ptr(), ic.data_ptr<int64_t>(), n, dw.data_ptr(), vocab, (int)cols, work.data_ptr<int>(), cur()),
+       "embed_grad");
+    return {dw, Tensor()};
+  }
+};
+
 }  // namespace
 
 void bind_model(py::module_& m) {
@@ -199,6 +225,8 @@ void bind_model(py::module_& m) {
     auto out = AddRmsNorm::apply(x, r, w, eps);
     return std::make_pair(out[0], out[1]);
   });
+  m.def("embedding", [](const Tensor& weight, const Tensor& ids) { return Embedding::apply(weight, ids); });
+  m.attr("EMBED_MAX_TOKENS") = oab::kEmbedMaxTokens;
   m.attr("NORM_MAX_COLS") = oab::kNormMaxCols;
   m.def("rope", [](const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
     auto out = Rope::apply(q, k, cos, sin);

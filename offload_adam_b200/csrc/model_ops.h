@@ -40,4 +40,13 @@ cudaError_t launch_rms_norm_grad(const void* g, const void* gsum, const void* x,
                                  void* dx, void* dw, float* partials, int64_t rows, int cols, cudaStream_t st);
 int rms_norm_partials(int64_t rows, int cols);
 
+// Gradient of an embedding table: dw (vocab, cols) = for every row the sum of the rows of
+// g (n, cols) whose ids name it, zero for the others.  cols % 8 == 0, n <= kEmbedMaxTokens,
+// vocab < 2^31; ids outside the table are ignored.  `work`: embed_work_ints(n, vocab) ints.
+// Sums in fp32, in a fixed order.
+constexpr int64_t kEmbedMaxTokens = 32768;
+int64_t embed_work_ints(int64_t n, int64_t vocab);
+cudaError_t launch_embed_grad(const void* g, const int64_t* ids, int64_t n, void* dw, int64_t vocab, int cols, int* work,
+                              cudaStream_t st);
+
 }  // namespace oab

@@ -123,6 +123,20 @@ def _apply_rope(x, cos, sin):
     return x * cos + rot * sin
 
 
+def _embed(module, ids):
+    """``module(ids)``; a training step's dense gradient of the table comes from one kernel
+    that also writes the zero rows.  Plain ``nn.Embedding`` without options, nobody watching."""
+    if type(module) is nn.Embedding:
+        w = module.weight
+        if (w.requires_grad and torch.is_grad_enabled() and use_kernels(w) and w.shape[1] % 8 == 0
+                and module.padding_idx is None and module.max_norm is None
+                and not (module.scale_grad_by_freq or module.sparse)
+                and type(ids) is torch.Tensor and ids.dtype == torch.int64 and ids.device == w.device
+                and ids.numel() <= _ext.load(required=True).EMBED_MAX_TOKENS and not _has_hooks(module)):
+            return _ext.load(required=True).embedding(w, ids)
+    return module(ids)
+
+
 class Attention(nn.Module):
     def __init__(self, cfg: LlamaConfig):
         super().__init__()
@@ -356,7 +370,7 @@ class LlamaForCausalLM(nn.Module):
         return self._rope[1], self._rope[2]
 
     def hidden_states(self, input_ids):
-        x = self.model.embed_tokens(input_ids)
+        x = _embed(self.model.embed_tokens, input_ids)
         cos, sin = self._rope_for(input_ids.shape[1], x.device, x.dtype)
         for layer in self.model.layers:
             if self.gradient_checkpointing and self.training:

@@ -159,3 +159,40 @@ def test_model_takes_the_torch_route_where_kernels_may_not_run():
     g, = torch.autograd.grad(model(ids).float().square().mean(), w, create_graph=False)
     assert g.isfinite().all()
     assert torch.func.jvp(lambda x: model.model.layers[0].mlp(x), (_rand(3, 256),), (_rand(3, 256),))[1].isfinite().all()
+
+
+# columns around a warp's 256; tokens around the order kernel's tile (2048) and its CTAs (64);
+# rows with none, some, more than 8 and all tokens; ids drawn from a few rows or all
+@pytest.mark.parametrize("cols", [8, 256, 264, 1000])
+@pytest.mark.parametrize("n,vocab,spread", [(1, 5, 5), (63, 1000, 1000), (65, 40, 3), (2049, 3001, 3001), (2048, 700, 1),
+                                            (5000, 131, 131)])
+def test_embedding_gradient(cols, n, vocab, spread):
+    C = _ext.load(required=True)
+    w = _rand(vocab, cols, seed=1).requires_grad_(True)
+    ids = torch.randint(0, spread, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    g = _rand(n, cols, seed=2)
+    y = C.embedding(w, ids)
+    assert torch.equal(y, w[ids])
+    y.backward(g)
+    want = torch.zeros(vocab, cols, device="cuda", dtype=torch.float64).index_add_(0, ids, g.double())
+    slack = 2.0 ** -20 * torch.zeros_like(want).index_add_(0, ids, g.double().abs())  # fp32 sums
+    assert ((w.grad.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + slack).all()
+
+
+def test_embedding_of_the_model_and_its_limits():
+    C = _ext.load(required=True)
+    model = build_llama(tiny_llama(tie_embeddings=False), device="cuda", seed=1)
+    ids = torch.randint(0, 1024, (2, 40), device="cuda")
+    table = model.model.embed_tokens.weight
+    out = []
+    for watched in (False, True):
+        if watched:  # a hook on the module: PyTorch's own gradient
+            model.model.embed_tokens.register_forward_hook(lambda m, i, o: None)
+        table.grad = None
+        n0 = C.launch_count()
+        model(ids, labels=ids).backward()
+        out.append((table.grad.clone(), C.launch_count() - n0))
+    assert out[0][1] == out[1][1] + 3
+    assert (out[0][0].float() - out[1][0].float()).norm() <= 1e-2 * out[1][0].float().norm()
+    with pytest.raises(RuntimeError):
+        C.embedding(table, torch.zeros(C.EMBED_MAX_TOKENS + 1, dtype=torch.int64, device="cuda"))
