@@ -479,6 +479,13 @@ int4_fake_quant_kernel(const T* x, int64_t nchunks, int lanes_per_group, T* out)
   }
 }
 
+// One item per thread, for kernels with nothing to set up and nothing to keep from item to
+// item: int8 14336 x 4096 to bf16 27 us (6.5 TB/s) where a grid of 8 CTAs per SM took 30, NVFP4
+// 23.5 and 25.  The NF4 kernel fills a table per CTA and gains nothing.
+unsigned grid_flat(int64_t work_items) {
+  const int64_t want = (work_items + kThreads - 1) / kThreads, cap = int64_t(1) << 30;
+  return (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
+}
 int grid_for(int64_t work_items) {
   int64_t want = (work_items + kThreads - 1) / kThreads;
   int cap = kNumSMs * 8;
@@ -531,7 +538,7 @@ cudaError_t launch_nvfp4_dequantize(const uint8_t* packed, const uint8_t* scales
   if (nb <= 0) return cudaSuccess;
   if (!aligned32(out) || (reinterpret_cast<uintptr_t>(packed) & 7u)) return cudaErrorInvalidValue;
   count_launch();
-  OAB_DISPATCH_IN(dtype, nvfp4_dequantize_kernel<T><<<grid_for(nb), kThreads, 0, st>>>(packed, scales, global_scale, nb, (T*)out));
+  OAB_DISPATCH_IN(dtype, nvfp4_dequantize_kernel<T><<<grid_flat(nb), kThreads, 0, st>>>(packed, scales, global_scale, nb, (T*)out));
   return cudaGetLastError();
 }
 
@@ -592,7 +599,7 @@ cudaError_t launch_int8_dequantize(const int8_t* q, const void* scales, int scal
                                    int64_t in_f, void* out, cudaStream_t st) {
   if (out_f <= 0) return cudaSuccess;
   count_launch();
-  OAB_DISPATCH_SCALE(scale_dtype, int8_dequantize_kernel<S><<<grid_for((out_f * in_f + 15) / 16), kThreads, 0, st>>>(q, (const S*)scales, out_f, in_f, (S*)out));
+  OAB_DISPATCH_SCALE(scale_dtype, int8_dequantize_kernel<S><<<grid_flat((out_f * in_f + 15) / 16), kThreads, 0, st>>>(q, (const S*)scales, out_f, in_f, (S*)out));
   return cudaGetLastError();
 }
 
