@@ -66,9 +66,9 @@ template <bool DECOUPLED, bool HAS_G2, bool PULL>
 __global__ void __launch_bounds__(kThreads, 2)
 adam_nf4_push_kernel(Ptrs t, Peers pr, int64_t n, AdamScalars s, const float* __restrict__ clip_ptr,
                      const int* abort_flag, Replicas q) {
-  __shared__ float lut[16];
+  __shared__ __align__(8) NF4Cell cells[kNF4Cells];
   if (abort_flag != nullptr && *reinterpret_cast<const volatile int*>(abort_flag) != 0) return;
-  if (threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
+  nf4_fill_cells(cells);
   __syncthreads();
   const float clip = clip_ptr ? *clip_ptr : 1.0f;
   const int lanes = q.group >> 4;
@@ -83,7 +83,7 @@ adam_nf4_push_kernel(Ptrs t, Peers pr, int64_t n, AdamScalars s, const float* __
     const float am = group_max(amax16(e), lanes);
     if (!live) continue;
     uint32_t w0, w1;
-    nf4_pack16(e, rcp_rn(fmaxf(am, kEps)), lut, w0, w1);
+    nf4_pack16(e, rcp_rn(fmaxf(am, kEps)), cells, w0, w1);
     const int64_t g = g0 + vec * 16;
     const bool first = (vec % lanes) == 0;
 #pragma unroll

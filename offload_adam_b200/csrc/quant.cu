@@ -126,7 +126,9 @@ template <typename T, bool FAKE>
 __global__ void __launch_bounds__(kThreads)
 nf4_quantize_kernel(const T* x, int64_t nchunks, int lanes_per_block, uint8_t* packed, float* absmax, T* out) {
   __shared__ float lut[16];
-  if (threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
+  __shared__ __align__(8) NF4Cell cells[kNF4Cells];
+  if (FAKE && threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
+  nf4_fill_cells(cells);
   __syncthreads();
   // grid covers whole warps so every shuffle has its partners
   const int64_t total = (nchunks + 31) / 32 * 32;
@@ -141,7 +143,7 @@ nf4_quantize_kernel(const T* x, int64_t nchunks, int lanes_per_block, uint8_t* p
     const float am = group_max(amax16(e), lanes_per_block);
     if (!live) continue;
     uint32_t w0, w1;
-    nf4_pack16(e, rcp_rn(fmaxf(am, kEps)), lut, w0, w1);
+    nf4_pack16(e, rcp_rn(fmaxf(am, kEps)), cells, w0, w1);
     if (FAKE) {
       nf4_unpack16(w0, w1, am, lut, e);
       Elem<T>::store16(out + c * 16, e);
