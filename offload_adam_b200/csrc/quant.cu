@@ -29,9 +29,9 @@ using namespace qm;
 // ------------------------------------------------------------------------ amax
 // partials[b] = max |x| over what CTA b read.  The reader of the partials reads x again:
 // plain loads leave in L2 what fits there (the streaming loads of the other kernels mark
-// their lines for eviction).  4096 x 4096 fp32 (67 MB): 8.3 us here and 11.1 us for the
-// quantization behind it; a call went from 30.7 us, with a fill and an atomic maximum, to
-// 27.4 us, which the host's part bounds.
+// their lines for eviction).  A call on 4096 x 4096 fp32 (67 MB) went from 30.7 us, with a fill
+// and an atomic maximum, to 27.4 us: about 13 us of DRAM reads here, 11 us for the
+// quantization out of L2, and the gap between the two.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) absmax_partials_kernel(const T* x, int64_t n, float* partials) {
   __shared__ float red[kThreads / 32];
@@ -482,8 +482,8 @@ int4_fake_quant_kernel(const T* x, int64_t nchunks, int lanes_per_group, T* out)
 }
 
 // One item per thread, for kernels with nothing to set up and nothing to keep from item to
-// item: int8 14336 x 4096 to bf16 27 us (6.5 TB/s) where a grid of 8 CTAs per SM took 30, NVFP4
-// 23.5 and 25.  The NF4 kernel fills a table per CTA and gains nothing.
+// item.  14336 x 4096 to bf16 between events, L2 cold: int8 33.3 us where a grid of 8 CTAs per
+// SM took 36.4, NVFP4 31.7 and 33.7.  The NF4 kernel fills a table per CTA and gains nothing.
 unsigned grid_flat(int64_t work_items) {
   const int64_t want = (work_items + kThreads - 1) / kThreads, cap = int64_t(1) << 30;
   return (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
