@@ -30,10 +30,10 @@ using namespace qm;
 // partials[b] = max |x| over what CTA b read.  The reader of the partials reads x again:
 // plain loads leave in L2 what fits there (the streaming loads of the other kernels mark
 // their lines for eviction).  A call on 4096 x 4096 fp32 (67 MB) went from 30.7 us, with a fill
-// and an atomic maximum, to 27.4 us: about 13 us of DRAM reads here, 11 us for the
+// and an atomic maximum, to 25.2 us: about 12 us of DRAM reads here, 11 us for the
 // quantization out of L2, and the gap between the two.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) absmax_partials_kernel(const T* x, int64_t n, float* partials) {
+__global__ void __launch_bounds__(kThreads, 8) absmax_partials_kernel(const T* x, int64_t n, float* partials) {
   __shared__ float red[kThreads / 32];
   float m = 0.f;
   const int64_t nvec = n >> 4;
@@ -60,12 +60,17 @@ __device__ __forceinline__ float tensor_amax(const float* amax, int n_amax, floa
   return red[0];
 }
 
+// 40 registers a thread: six CTAs fit an SM, and the grid is no larger (two more per SM ran
+// as a second, mostly empty wave; with that and eight CTAs per SM in the pass for the maximum,
+// which had room for five, a call took 27.4 us instead of 25.2).
+constexpr int kNVFP4PerSM = 6;
+
 // One thread per 16-element block, from the end of the tensor to its start: a pass for the
 // maximum has just read it forwards, and its end is what L2 still holds.  The four scale bytes of four neighbouring blocks
 // are combined with shuffles and leave as one 32-bit store; global_scale[0] is written
 // by thread 0.  FAKE: instead of the payload, write the de-quantized values to `out`.
 template <typename T, bool FAKE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kNVFP4PerSM)
 nvfp4_quantize_kernel(const T* x, int64_t nblocks, const float* amax, int n_amax, uint8_t* packed, uint8_t* scales,
                       float* global_scale_out, int scale_words_ok, T* out) {
   __shared__ float red[kThreads / 32];
@@ -123,7 +128,7 @@ nvfp4_dequantize_kernel(const uint8_t* packed, const uint8_t* scales, const floa
 // one thread per 16 elements; lanes_per_block = blocksize / 16 (power of two <= 32).
 // FAKE: write the de-quantized values to `out` instead of the payload.
 template <typename T, bool FAKE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 8)
 nf4_quantize_kernel(const T* x, int64_t nchunks, int lanes_per_block, uint8_t* packed, float* absmax, T* out) {
   __shared__ float lut[16];
   __shared__ __align__(8) NF4Cell cells[kNF4Cells];
@@ -488,9 +493,9 @@ unsigned grid_flat(int64_t work_items) {
   const int64_t want = (work_items + kThreads - 1) / kThreads, cap = int64_t(1) << 30;
   return (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
 }
-int grid_for(int64_t work_items) {
+int grid_for(int64_t work_items, int per_sm = 8) {
   int64_t want = (work_items + kThreads - 1) / kThreads;
-  int cap = kNumSMs * 8;
+  int cap = kNumSMs * per_sm;
   return (int)(want < 1 ? 1 : (want > cap ? cap : want));
 }
 
@@ -529,7 +534,7 @@ cudaError_t launch_nvfp4_quantize(const void* x, int dtype, int64_t numel, const
   if (!aligned32(x) || (reinterpret_cast<uintptr_t>(packed) & 7u)) return cudaErrorInvalidValue;
   const int words_ok = (reinterpret_cast<uintptr_t>(scales) & 3u) == 0;
   count_launch();
-  OAB_DISPATCH_IN(dtype, nvfp4_quantize_kernel<T, false><<<grid_for(nb), kThreads, 0, st>>>(
+  OAB_DISPATCH_IN(dtype, nvfp4_quantize_kernel<T, false><<<grid_for(nb, kNVFP4PerSM), kThreads, 0, st>>>(
       (const T*)x, nb, amax, n_amax, packed, scales, global_scale, words_ok, nullptr));
   return cudaGetLastError();
 }
@@ -641,7 +646,7 @@ cudaError_t launch_fake_quant(int format, const void* x, void* out, int dtype, i
     case kQNVFP4: {
       if (in_f % 16 != 0 || tensor_amax == nullptr || !aligned32(x) || !aligned32(out)) return cudaErrorInvalidValue;
       const int64_t nb = numel / 16;
-      OAB_DISPATCH_IN(dtype, nvfp4_quantize_kernel<T, true><<<grid_for(nb), kThreads, 0, st>>>(
+      OAB_DISPATCH_IN(dtype, nvfp4_quantize_kernel<T, true><<<grid_for(nb, kNVFP4PerSM), kThreads, 0, st>>>(
           (const T*)x, nb, tensor_amax, n_amax, nullptr, nullptr, nullptr, 0, (T*)out));
       break;
     }
