@@ -7,9 +7,10 @@ reference's example trainer offers Liger's fused linear cross-entropy for this, 
 for Qwen3 only (reference: examples/e2e_train/train.py:76-115).  ``causal_lm_loss`` does
 the same for any HF causal LM that exposes its decoder as ``.model`` and an unbiased
 ``nn.Linear`` ``.lm_head`` (Llama, Qwen2/3, Mistral, Gemma, ...): the decoder runs as
-usual, the head and the loss run chunk by chunk through
-:func:`offload_adam_b200.models.llama.chunked_linear_cross_entropy`, which forms the
-gradients of the hidden states and of the head weight in the same pass.  Tied
+usual, the head and the loss run a group of rows at a time through
+:func:`offload_adam_b200.models.llama.chunked_linear_cross_entropy`, which keeps at most
+three chunks of bf16 logits for the gradients of the hidden states and of the head
+weight.  Tied
 embeddings work unchanged (the head weight is the embedding parameter; autograd adds
 both contributions)."""
 

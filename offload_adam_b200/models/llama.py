@@ -6,7 +6,7 @@ attention, gradient checkpointing and a fused linear cross-entropy
 ingredients without external model code: RMSNorm, rotary embeddings, grouped
 query attention through ``scaled_dot_product_attention``, SwiGLU, optional
 per-layer activation checkpointing and a chunked linear + cross-entropy head
-that never materialises the full ``(tokens, vocab)`` logits.
+that holds the logits of a few thousand tokens at most, in bf16.
 
 Parameter names and shapes match the HF Llama layout (``model.embed_tokens``,
 ``model.layers.N.self_attn.{q,k,v,o}_proj``, ``mlp.{gate,up,down}_proj``,
@@ -40,7 +40,7 @@ class LlamaConfig:
     rms_eps: float = 1e-5
     tie_embeddings: bool = False
     init_std: float = 0.02
-    ce_chunk: int = 2048  # rows of the logits computed at a time by the loss head
+    ce_chunk: int = 2048  # rows of the logits that the loss head holds (see _CE_ROWS_PER_CHUNK)
     head_dim_override: Optional[int] = None  # Qwen3: 128 whatever hidden_size / num_heads is
     qk_norm: bool = False  # Qwen3: RMSNorm over head_dim on queries and keys before RoPE
 
