@@ -27,4 +27,10 @@ cudaError_t launch_ce_grad(const void* logits, int64_t pitch, const int64_t* lab
                            const float* row_max, const float* row_inv_sum, const float* inv, const float* g,
                            void* grad, cudaStream_t st);
 
+// Sum of bf16 tensors in fp32, one after another: value = acc + g with acc bf16
+// (acc_is_f32 false) or fp32; written to out_f32 (may be acc) or, rounded, to out_bf16.
+// All 32-byte aligned.
+cudaError_t launch_sum_bf16(const void* acc, bool acc_is_f32, const void* g, float* out_f32, void* out_bf16, int64_t n,
+                            cudaStream_t st);
+
 }  // namespace oab

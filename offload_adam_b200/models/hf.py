@@ -9,7 +9,7 @@ the same for any HF causal LM that exposes its decoder as ``.model`` and an unbi
 ``nn.Linear`` ``.lm_head`` (Llama, Qwen2/3, Mistral, Gemma, ...): the decoder runs as
 usual, the head and the loss run a group of rows at a time through
 :func:`offload_adam_b200.models.llama.chunked_linear_cross_entropy`, which keeps at most
-three chunks of bf16 logits for the gradients of the hidden states and of the head
+four chunks of bf16 logits for the gradients of the hidden states and of the head
 weight.  Tied
 embeddings work unchanged (the head weight is the embedding parameter; autograd adds
 both contributions)."""

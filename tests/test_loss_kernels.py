@@ -5,6 +5,7 @@ import math
 import pytest
 import torch
 
+from offload_adam_b200 import _ext
 from offload_adam_b200.models import llama
 from offload_adam_b200.models.llama import chunked_linear_cross_entropy
 
@@ -42,7 +43,7 @@ def _rel(a, b):
 # vocabularies around a 16-value vector, a pair of vectors per thread and the CTA sizes;
 # rows in one group, in several and a ragged last one
 @pytest.mark.parametrize("vocab", [1, 15, 16, 17, 1000, 4095, 8192, 8193, 32003, 128256])
-@pytest.mark.parametrize("n,chunk", [(1, 128), (37, 128), (300, 50)])
+@pytest.mark.parametrize("n,chunk", [(1, 128), (37, 128), (300, 50), (300, 15)])
 def test_linear_cross_entropy_matches_fp64(vocab, n, chunk):
     h, w, labels = _inputs(n, 64, vocab)
     got = _run(chunked_linear_cross_entropy, h, w, labels, chunk, g=0.25)
@@ -58,6 +59,17 @@ def test_linear_cross_entropy_matches_fp64(vocab, n, chunk):
         # worse than the PyTorch route
         assert _rel(got[k], want[k]) <= 3 * 2.0 ** -8
         assert _rel(got[k], want[k]) <= 1.1 * _rel(old[k], want[k]) + 1e-4
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 4096, 4113])
+def test_sum_of_bf16_tensors(n):
+    C = _ext.load(required=True)
+    a, b, c = (torch.randn(n, device="cuda").to(torch.bfloat16) for _ in range(3))
+    ab = C.sum_bf16(a, b, False)
+    assert torch.equal(ab, a.float() + b.float())
+    assert torch.equal(C.sum_bf16(a, b, True), (a.float() + b.float()).to(torch.bfloat16))
+    assert torch.equal(C.sum_bf16(ab, c, True), (a.float() + b.float() + c.float()).to(torch.bfloat16))
+    assert torch.equal(C.sum_bf16(ab, c, False), a.float() + b.float() + c.float())
 
 
 def test_loss_without_gradient_and_all_ignored():
