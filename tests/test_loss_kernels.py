@@ -48,7 +48,8 @@ def test_linear_cross_entropy_matches_fp64(vocab, n, chunk):
     h, w, labels = _inputs(n, 64, vocab)
     got = _run(chunked_linear_cross_entropy, h, w, labels, chunk, g=0.25)
     want = _fp64(h, w, labels, g=0.25)
-    old = _run(llama._ChunkedLinearCE.apply, h, w, labels, chunk, g=0.25)
+    # the PyTorch route on as many rows at a time: the library sees the same products
+    old = _run(llama._ChunkedLinearCE.apply, h, w, labels, chunk * llama._CE_ROWS_PER_CHUNK, g=0.25)
     # bf16 logits round by up to 2^-8 of their value, a few units here
     assert abs(got[0] - want[0]) <= 2.0 ** -8 * max(1.0, abs(want[0].item()))
     for k in (1, 2):
