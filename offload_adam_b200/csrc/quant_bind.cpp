@@ -184,48 +184,56 @@ Tensor qgemv(const Packed& w, const Tensor& x, const Tensor& bias) {
   return y;
 }
 
-// (The Python node cost 60 us more per forward and backward: 333 tokens through 2816 x 1024
-// int4 with bias, 35 us of kernels, took 202 us and takes 135.)
-//
-// y = x W^T + b.  `weight` is the wrapper that autograd knows; the packed tensors travel
-// beside it.  As in the Python node for the other calls, backward decodes the payload as it
-// is then, and its products are ordinary operations (they can be differentiated again).
+// The weight as backward finds it.  The Python object is asked for its payload, as the Python
+// node does: a saved-tensor hook may have returned another weight than forward had, or a
+// dense tensor.
+Tensor dense_weight(const Tensor& weight, at::ScalarType dtype) {
+  at::NoGradGuard no_grad;
+  Packed w;
+  {
+    py::gil_scoped_acquire gil;
+    try {
+      const py::object o = py::cast(weight);
+      if (!py::hasattr(o, "KERNEL_PAYLOAD")) return weight.to(dtype);
+      const py::tuple names = o.attr("KERNEL_PAYLOAD");
+      w.format = o.attr("KERNEL_FORMAT").cast<int64_t>();
+      w.group = o.attr("kernel_group")().cast<int64_t>();
+      w.packed = o.attr(py::object(names[0])).cast<Tensor>();
+      w.scales = o.attr(py::object(names[1])).cast<Tensor>();
+      if (w.format == oab::kQNVFP4) w.global_scale = o.attr("global_scale").cast<Tensor>();
+      if (!w.packed.is_cuda() || !packed_ok(w, w.packed.device()))
+        return o.attr("dequantize")(py::cast(dtype)).cast<Tensor>();
+    } catch (const py::error_already_set& e) {
+      TORCH_CHECK(false, e.what());
+    }
+  }
+  c10::cuda::CUDAGuard guard(w.packed.device());
+  return packed_dense(w).to(dtype);
+}
+
+// y = x W^T + b.  `weight` is the wrapper that autograd knows; its packed tensors travel
+// beside it.  It is saved as an input is: changing it in place before backward is an error,
+// and saved-tensor hooks see it.  The products of backward are ordinary operations (they can
+// be differentiated again).  333 tokens through 2816 x 1024 int4 with bias, forward and
+// backward, a whole call (35 us of kernels): 189 us with the Python node, 135 with this one.
 struct QLinear : torch::autograd::Function<QLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias, const Packed& w) {
     c10::cuda::CUDAGuard guard(x.device());
-    ctx->save_for_backward({x});
-    ctx->saved_data["packed"] = w.packed;
-    ctx->saved_data["scales"] = w.scales;
-    if (w.global_scale.defined()) ctx->saved_data["global_scale"] = w.global_scale;
-    ctx->saved_data["format"] = w.format;
-    ctx->saved_data["group"] = w.group;
+    ctx->save_for_backward({x, weight});
     ctx->saved_data["bias"] = bias.has_value() && bias->defined();
     const Tensor b = bias.has_value() ? *bias : Tensor();
     const Tensor few = qgemv(w, x, b);
     return few.defined() ? few : at::linear(x, packed_dense(w), bias);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor x = ctx->get_saved_variables()[0], &gy = grads[0];
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &weight = saved[1], &gy = grads[0];
     if (!gy.defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
-    Packed w;
-    w.format = ctx->saved_data["format"].toInt();
-    w.group = ctx->saved_data["group"].toInt();
-    w.packed = ctx->saved_data["packed"].toTensor();
-    w.scales = ctx->saved_data["scales"].toTensor();
-    if (w.format == oab::kQNVFP4) w.global_scale = ctx->saved_data["global_scale"].toTensor();
-    c10::cuda::CUDAGuard guard(w.packed.device());
-    TORCH_CHECK(packed_ok(w, w.packed.device()), "the packed weight changed its layout between forward and backward");
-    const Tensor g2 = gy.reshape({-1, w.rows});
+    c10::cuda::CUDAGuard guard(gy.device());
+    const Tensor g2 = gy.reshape({-1, weight.size(0)});
     Tensor gx, gw, gb;
-    if (ctx->needs_input_grad(0)) {
-      Tensor dense;
-      {
-        at::NoGradGuard no_grad;
-        dense = packed_dense(w);
-      }
-      gx = g2.mm(dense.to(gy.scalar_type())).view(x.sizes());
-    }
-    if (ctx->needs_input_grad(1)) gw = g2.t().mm(x.reshape({-1, w.cols}));
+    if (ctx->needs_input_grad(0)) gx = g2.mm(dense_weight(weight, gy.scalar_type())).view(x.sizes());
+    if (ctx->needs_input_grad(1)) gw = g2.t().mm(x.reshape({-1, weight.size(1)}));
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) gb = g2.sum(0);
     return {gx, gw, gb, Tensor()};
   }

@@ -133,3 +133,37 @@ def test_autograd_node_with_frozen_inputs_and_second_derivative():
     g1, = torch.autograd.grad(z.sum(), x)
     g2, = torch.autograd.grad(F.linear(x, trained).sum(), x)
     assert torch.equal(g1, g2)
+
+
+@pytest.mark.parametrize("cls,kw", [(NVFP4QWeight, {}), (NF4QWeight, {}), (Int4QWeight, {}), (Int8QWeight, {})])
+@pytest.mark.parametrize("tokens", [1, 20])
+def test_weight_changed_in_place_before_backward_is_an_error(cls, kw, tokens):
+    """As for a dense weight: the gradient would belong to another weight than the result."""
+    w, x, _ = _case(cls, 64, 128, tokens, False, **kw)
+    x.requires_grad_(True)
+    y = F.linear(x, w)
+    with torch.no_grad():
+        w.copy_(torch.ones(64, 128, device="cuda", dtype=torch.bfloat16))
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
+
+
+@pytest.mark.parametrize("cls,kw", [(NVFP4QWeight, {}), (NF4QWeight, {}), (Int4QWeight, {}), (Int8QWeight, {})])
+def test_saved_tensor_hooks_see_the_weight(cls, kw):
+    w, x, _ = _case(cls, 64, 128, 20, False, **kw)
+    other, _, _ = _case(cls, 64, 128, 21, False, **kw)
+    x.requires_grad_(True)
+    seen = []
+
+    def pack(t):
+        seen.append(t)
+        return t
+
+    # backward uses what the hook returns: another packed weight, or a dense one
+    for back, want in ((lambda t: other.data, other), (lambda t: t.detach().dequantize(), w)):
+        seen.clear()
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: back(t) if isinstance(t, cls) else t):
+            y = F.linear(x, w)
+            gx, = torch.autograd.grad(y.sum(), x)
+        assert any(isinstance(t, cls) for t in seen)
+        assert torch.equal(gx, torch.ones_like(y) @ want.data.dequantize(torch.bfloat16))
