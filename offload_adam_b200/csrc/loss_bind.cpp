@@ -84,14 +84,18 @@ void ce_grad(const Tensor& logits, const Tensor& labels, const Tensor& stats, co
                          inv.data_ptr<float>(), gp, grad.data_ptr(), cur()), "ce_grad");
 }
 
-// fp32(acc) + fp32(g), in fp32 (into `acc` when it is fp32) or rounded to bf16; g is bf16
-Tensor sum_bf16(const Tensor& acc, const Tensor& g, bool round) {
+// fp32(acc) + fp32(g), in fp32 (into `acc` when it is fp32) or rounded to bf16 (into `to` when
+// it is given; it may be g); g is bf16
+Tensor sum_bf16(const Tensor& acc, const Tensor& g, bool round, const std::optional<Tensor>& to) {
   TORCH_CHECK(acc.is_cuda() && g.device() == acc.device() && acc.is_contiguous() && g.is_contiguous() && acc.sizes() == g.sizes() &&
                   g.scalar_type() == at::kBFloat16 && (acc.scalar_type() == at::kBFloat16 || acc.scalar_type() == at::kFloat),
               "sum_bf16: contiguous CUDA tensors of one shape");
   c10::cuda::CUDAGuard guard(acc.device());
   const bool f32 = acc.scalar_type() == at::kFloat;
-  Tensor out = round ? at::empty_like(g) : (f32 ? acc : at::empty(g.sizes(), g.options().dtype(at::kFloat)));
+  const bool given = round && to.has_value() && to->defined();
+  TORCH_CHECK(!given || (to->sizes() == g.sizes() && to->scalar_type() == at::kBFloat16 && to->is_contiguous() && to->device() == g.device()),
+              "sum_bf16: `to` like g");
+  Tensor out = given ? *to : round ? at::empty_like(g) : (f32 ? acc : at::empty(g.sizes(), g.options().dtype(at::kFloat)));
   ok(oab::launch_sum_bf16(acc.data_ptr(), f32, g.data_ptr(), round ? nullptr : out.data_ptr<float>(),
                           round ? out.data_ptr() : nullptr, g.numel(), cur()), "sum_bf16");
   return out;
@@ -103,7 +107,7 @@ void bind_loss(py::module_& m) {
   m.def("ce_logits_buffer", &ce_logits_buffer);
   m.def("ce_stats", &ce_stats);
   m.def("ce_finish", &ce_finish, py::arg("row_loss"), py::arg("labels"), py::arg("loss"), py::arg("inv"));
-  m.def("sum_bf16", &sum_bf16);
+  m.def("sum_bf16", &sum_bf16, py::arg("acc"), py::arg("g"), py::arg("round"), py::arg("to") = py::none());
   m.def("ce_grad", &ce_grad, py::arg("logits"), py::arg("labels"), py::arg("stats"), py::arg("inv"), py::arg("g"),
         py::arg("grad"));
 }

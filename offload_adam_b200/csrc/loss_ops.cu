@@ -183,7 +183,7 @@ ce_grad_kernel(const uint16_t* logits, int64_t pitch, const int64_t* __restrict_
 // with the adds, 41.3 ms now; 8192 tokens, which now are one group, 24.0 and 19.0 ms.
 template <bool ACC32, bool OUT32>
 __global__ void __launch_bounds__(kGradThreads)
-sum_bf16_kernel(const void* acc, const uint16_t* __restrict__ g, float* out32, uint16_t* out16, int64_t n) {
+sum_bf16_kernel(const void* acc, const uint16_t* g, float* out32, uint16_t* out16, int64_t n) {
   const int64_t i = ((int64_t)blockIdx.x * kGradThreads + threadIdx.x) * 16;
   if (i >= n) return;
   if (i + 16 > n) {

@@ -239,20 +239,35 @@ class _ChunkedLinearCE(torch.autograd.Function):
 
 
 # Rows of the logits that the kernel route handles at a time, in units of the caller's chunk.
-# The torch route holds 12 bytes for every logit of a chunk (bf16, fp32, fp32 probabilities,
-# their bf16 image) next to 6 bytes for every weight of the head (fp32 gradient, bf16
-# product); the kernel route holds bf16 logits and, in backward, their bf16 gradient: 4 bytes
-# for up to four times the rows, and nothing else.
+# With c rows a chunk, V words and hidden size H, the PyTorch route's peak is the larger of
+# 16 c V + 4 V H bytes (two chunks' logits in fp32 and bf16, the fp32 gradient of the head) and
+# 10 c V + 6 V H (one chunk, and a product that is added).  Here one group of R rows takes
+# 4 R V + 2 V H (bf16 logits and their gradient, the gradient of the head), several groups
+# 2 R V + 6 V H: R = 4 c stays below it for every H.  Measured for 4096 rows, c = 2048, hidden
+# 1024, 128256 words: 2.2 GB, PyTorch route 4.7; 20000 rows, hidden 256, 32000 words: 0.6 and 1.1.
 _CE_ROWS_PER_CHUNK = 4
 
 
-def _product_operand(d, hidden):
-    """The gradient of the logits as its two products read it.  The library reduces split sums
-    of aligned operands in bf16 where the result has too few tiles for the chip (0.9 % error in
-    the hidden states' gradient of 60 rows of a 32003-word vocabulary, 0.26 % from unaligned
-    rows); there, the packed rows that the PyTorch route has keep its precision."""
-    small = d.shape[0] * hidden < 148 * 128 * 256
-    return d.contiguous() if d.shape[1] % 8 and small else d
+def _head_logits(h, weight, out, chunk):
+    """``out = h @ weight.T``.  A vocabulary that is no multiple of 8 takes the library's
+    kernels for unaligned operands, which may split a sum and add its parts in bf16; how many
+    rows there are decides it.  Those take the caller's chunk (840 x 32003: 0.17 % off 64 bits
+    for 2048 rows at a time, 0.20 % for 8192)."""
+    step = chunk if weight.shape[0] % 8 else h.shape[0]
+    for s in range(0, h.shape[0], step):
+        torch.mm(h[s:s + step], weight.T, out=out[s:s + step])
+
+
+def _hidden_grad(d, weight, out, rows):
+    """``out = d @ weight``.  For the same vocabularies the sum over the words is kept in fp32
+    to its end, ``rows`` rows at a time: split sums in bf16 left 0.2 to 1 % of error (60 rows of
+    32003 words, hidden 64: 0.57 %), fp32 leaves the 0.17 % of the one rounding, in the same
+    time (32003 x 840, 8192 rows: 3656 us, 3645 in bf16)."""
+    if d.shape[1] % 8 == 0:
+        torch.mm(d, weight, out=out)
+        return
+    for s in range(0, d.shape[0], rows):
+        out[s:s + rows] = torch.mm(d[s:s + rows], weight, out_dtype=torch.float32)
 
 
 class _KernelLinearCE(torch.autograd.Function):
@@ -276,7 +291,7 @@ class _KernelLinearCE(torch.autograd.Function):
         logits = C.ce_logits_buffer(h, min(N, rows), V)
         stats = torch.empty(3 * logits.shape[0], **f32)
         if ctx.one_group:
-            torch.mm(h, weight.T, out=logits)
+            _head_logits(h, weight, logits, chunk)
             C.ce_stats(logits, labels, stats)
             C.ce_finish(stats[2 * N:], labels, loss, inv)
             if ctx.want_grad:
@@ -290,15 +305,18 @@ class _KernelLinearCE(torch.autograd.Function):
         for s in range(0, N, rows):
             n = min(N - s, rows)
             hs, lab, lo, st = h[s:s + n], labels[s:s + n], logits[:n], stats[:3 * n]
-            torch.mm(hs, weight.T, out=lo)
+            _head_logits(hs, weight, lo, chunk)
             C.ce_stats(lo, lab, st)
             row_loss[s:s + n] = st[2 * n:]
             if ctx.want_grad:
                 C.ce_grad(lo, lab, st, inv, None, lo)
-                d = _product_operand(lo, h.shape[1])
-                torch.mm(d, weight, out=gh[s:s + n])
-                part = d.T @ hs
-                gw = part if gw is None else C.sum_bf16(gw, part, s + rows >= N)  # fp32 until the last
+                _hidden_grad(lo, weight, gh[s:s + n], max(V // 2, 128))
+                if gw is None:  # fp32 until the last; two groups are one sum
+                    gw = lo.T @ hs if N <= 2 * rows else torch.mm(lo.T, hs, out_dtype=torch.float32)
+                else:
+                    part = lo.T @ hs
+                    gw = C.sum_bf16(gw, part, s + rows >= N, part)
+                    del part  # or it lives beside the next one
         C.ce_finish(row_loss, labels, loss, inv)
         if ctx.want_grad:
             ctx.save_for_backward(gh, gw)
@@ -311,6 +329,7 @@ class _KernelLinearCE(torch.autograd.Function):
             return gh * g.to(gh.dtype), gw * g.to(gw.dtype), None, None
         C = _ext.load(required=True)
         h, weight, labels, logits, stats, inv = ctx.saved_tensors
+        V = weight.shape[0]
         through = g.requires_grad and torch.is_grad_enabled()  # keep the graph through g
         # saved-tensor hooks may have returned copies without the padded rows
         if logits.stride(0) % 16 or logits.data_ptr() % 32 or not _whole_vectors(logits):
@@ -318,9 +337,12 @@ class _KernelLinearCE(torch.autograd.Function):
         d = C.ce_logits_buffer(logits, *logits.shape)
         with torch.no_grad():
             C.ce_grad(logits, labels, stats, inv, None if through else g.detach().float().contiguous(), d)
-            d = _product_operand(d, h.shape[1])
-            gh = d @ weight if ctx.needs_input_grad[0] else None
-            gw = d.T @ h if ctx.needs_input_grad[1] else None
+            gh = gw = None
+            if ctx.needs_input_grad[0]:
+                gh = torch.empty_like(h)
+                _hidden_grad(d, weight, gh, max(V, 128))
+            if ctx.needs_input_grad[1]:
+                gw = d.T @ h
         if through:
             gh = None if gh is None else gh * g.to(gh.dtype)
             gw = None if gw is None else gw * g.to(gw.dtype)
@@ -336,6 +358,7 @@ def _whole_vectors(x):
 
 def chunked_linear_cross_entropy(h, weight, labels, chunk=2048):
     kernels = (use_kernels(h, weight) and h.dim() == 2 and weight.dim() == 2 and h.numel() > 0 and weight.numel() > 0
+               and h.shape[1] % 8 == 0  # all operands of the products would be unaligned
                and type(labels) is torch.Tensor and labels.is_cuda and labels.dtype == torch.int64
                and labels.shape == h.shape[:1] and h.device == weight.device == labels.device)
     if kernels:

@@ -48,8 +48,7 @@ def test_linear_cross_entropy_matches_fp64(vocab, n, chunk):
     h, w, labels = _inputs(n, 64, vocab)
     got = _run(chunked_linear_cross_entropy, h, w, labels, chunk, g=0.25)
     want = _fp64(h, w, labels, g=0.25)
-    # the PyTorch route on as many rows at a time: the library sees the same products
-    old = _run(llama._ChunkedLinearCE.apply, h, w, labels, chunk * llama._CE_ROWS_PER_CHUNK, g=0.25)
+    old = _run(llama._ChunkedLinearCE.apply, h, w, labels, chunk, g=0.25)
     # bf16 logits round by up to 2^-8 of their value, a few units here
     assert abs(got[0] - want[0]) <= 2.0 ** -8 * max(1.0, abs(want[0].item()))
     for k in (1, 2):
@@ -62,6 +61,33 @@ def test_linear_cross_entropy_matches_fp64(vocab, n, chunk):
         assert _rel(got[k], want[k]) <= 1.1 * _rel(old[k], want[k]) + 1e-4
 
 
+# products large enough for the library to split: few tiles, long sums, vocabularies of every
+# alignment; one group of rows, two, and several
+@pytest.mark.parametrize("vocab,hidden,n,chunk", [(1001, 2048, 4096, 2048), (1001, 256, 8192, 1024), (32003, 64, 60, 15),
+                                                  (32003, 64, 4096, 256), (32003, 840, 3000, 512), (32004, 256, 3000, 512),
+                                                  (32000, 256, 3000, 512), (5001, 512, 777, 64), (8192, 1024, 600, 128),
+                                                  (1001, 100, 300, 64)])
+def test_no_less_precise_and_no_larger_than_the_pytorch_route(vocab, hidden, n, chunk):
+    """At the chunk that the caller passes."""
+    h, w, labels = _inputs(n, hidden, vocab)
+    want = _fp64(h, w, labels)
+    got, old, peak = [], [], []
+    for fn, out in ((chunked_linear_cross_entropy, got), (llama._ChunkedLinearCE.apply, old)):
+        for turn in range(2):  # the library takes its workspace in the first
+            a = b = None
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            a, b = h.detach().requires_grad_(True), w.detach().requires_grad_(True)
+            fn(a, b, labels, chunk).backward()
+            peak.append(torch.cuda.max_memory_allocated() - before)
+        out += [a.grad.double(), b.grad.double()]
+        del a, b
+    for k in (0, 1):
+        assert _rel(got[k], want[k + 1]) <= 1.1 * _rel(old[k], want[k + 1]) + 1e-4
+    # labels' statistics (three floats a row) and 512-byte blocks of the allocator on top
+    assert peak[1] <= peak[3] + 16 * n + 16384
+
+
 @pytest.mark.parametrize("n", [1, 15, 16, 4096, 4113])
 def test_sum_of_bf16_tensors(n):
     C = _ext.load(required=True)
@@ -70,6 +96,9 @@ def test_sum_of_bf16_tensors(n):
     assert torch.equal(ab, a.float() + b.float())
     assert torch.equal(C.sum_bf16(a, b, True), (a.float() + b.float()).to(torch.bfloat16))
     assert torch.equal(C.sum_bf16(ab, c, True), (a.float() + b.float() + c.float()).to(torch.bfloat16))
+    into = c.clone()
+    assert C.sum_bf16(ab, into, True, into) is into
+    assert torch.equal(into, (a.float() + b.float() + c.float()).to(torch.bfloat16))
     assert torch.equal(C.sum_bf16(ab, c, False), a.float() + b.float() + c.float())
 
 
