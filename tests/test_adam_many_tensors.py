@@ -81,3 +81,31 @@ def test_empty_parameters_are_passed_over(mode):
             p.grad = torch.ones_like(p)
         opt.step()
     assert all((p < 1).all() for p in ps) and [opt.state[p]["step"] for p in ps] == [2, 2, 2]
+
+
+@pytest.mark.parametrize("mode", list(STATE_DTYPES))
+@pytest.mark.parametrize("shared", ["parameter", "state", "gradient"])
+def test_tensors_that_share_memory_are_stepped_in_order(mode, shared):
+    """A launch over both would update the same elements twice at once."""
+    def make():
+        a, b, c = _items(mode, [300_000, 200_000, 100_000], 0)
+        if shared == "parameter":
+            b = (a[0][100_000:], *b[1:]) if b[0] is not None else b
+        elif shared == "state":
+            b[1]["exp_avg"] = a[1]["exp_avg"][:200_000]
+        else:  # written by a, read by b
+            b[1]["grad"] = a[0][50_000:250_000]
+        return [a, b, c]
+
+    one, many = make(), make()
+    hp = (1e-2, 0.1, 0.9, 0.99, 1e-8, 3)
+    for p, st, seed in one:
+        adam_step(mode, p, st, *hp, seed=seed)
+    C = _ext.load(required=True)
+    n0 = C.launch_count()
+    adam_step_many(mode, many, *hp)
+    assert C.launch_count() - n0 == 3
+    for (p, a, _), (q, b, _) in zip(one, many):
+        assert p is None or torch.equal(p, q)
+        for k in a:
+            assert torch.equal(a[k], b[k])
