@@ -228,10 +228,10 @@ cudaError_t launch_adam_step_many(ManyEntry* entries, int count, int mode, bool 
     int64_t total = 0;
     for (int i = at; i < count && i < at + kManyTensors; ++i) {
       const ManyEntry& e = entries[i];
-      if (e.n <= 0) continue;  // before the checks: an empty tensor has no address
       if (e.g == nullptr || e.m == nullptr || e.v == nullptr) return cudaErrorInvalidValue;
       if (mode != kModeFP32Master && e.p == nullptr) return cudaErrorInvalidValue;
       if (mode != kModeSR && e.extra == nullptr) return cudaErrorInvalidValue;
+      if (e.n <= 0) continue;
       total += e.n;
       ManyEntry& o = t.e[t.count++];
       o = e;

@@ -73,17 +73,6 @@ def test_optimizer_with_uneven_step_counts():
 
 
 @pytest.mark.parametrize("mode", list(STATE_DTYPES))
-def test_empty_parameters_are_passed_over(mode):
-    ps = [torch.nn.Parameter(torch.ones(n, device="cuda", dtype=torch.bfloat16)) for n in (17, 0, 5)]
-    opt = Adam(ps, lr=1e-2, mode=mode)
-    for _ in range(2):
-        for p in ps:
-            p.grad = torch.ones_like(p)
-        opt.step()
-    assert all((p < 1).all() for p in ps) and [opt.state[p]["step"] for p in ps] == [2, 2, 2]
-
-
-@pytest.mark.parametrize("mode", list(STATE_DTYPES))
 @pytest.mark.parametrize("shared", ["parameter", "state", "gradient"])
 def test_tensors_that_share_memory_are_stepped_in_order(mode, shared):
     """A launch over both would update the same elements twice at once."""
