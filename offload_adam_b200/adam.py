@@ -16,7 +16,7 @@ import torch
 from torch.optim.optimizer import Optimizer
 
 from ._master import MasterLoadingMixin, is_quant
-from .ops.adam_step import STEP_FNS, adam_step_many
+from .ops.adam_step import MANY_TENSORS, STEP_FNS, adam_step_many
 
 STATE_DTYPES = {
     "stochastic_rounding": {"exp_avg": torch.bfloat16, "exp_avg_sq": torch.bfloat16},
@@ -94,47 +94,69 @@ class Adam(MasterLoadingMixin, Optimizer):
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
+        states, with_seed = self.config["states"], self.mode == "stochastic_rounding"
         for group in self.param_groups:
-            pending = {}  # step count -> CUDA parameters due, in one launch together
-            for p in group["params"]:
-                grad = p.grad
-                if grad is None:
-                    continue
-                if grad.is_sparse:
-                    self._step_pending(group, pending)
-                    raise RuntimeError("Sparse gradient is not supported")
-                state = self.state[p]
-                self._init_state_if_empty(p, state)
-                state["step"] += 1
-                quant = is_quant(p)
-                if quant:
-                    self._warn_lossy_master_once(state)
-                tensors = {k: state[k] for k in self.config["states"]}
-                tensors["grad"] = grad if grad.dtype == torch.bfloat16 else grad.to(torch.bfloat16)
-                seed = self._rng.getrandbits(63) if self.mode == "stochastic_rounding" else 0
-                # a quantized weight has no bf16 image to write: only the master moves,
-                # then copy_ re-quantizes the packed payload from it
-                pending.setdefault(state["step"], []).append((p, quant, tensors, seed))
-            self._step_pending(group, pending)
+            due = []  # CUDA parameters of one step count, which the next launch takes
+            try:
+                for p in group["params"]:
+                    grad = p.grad
+                    if grad is None:
+                        continue
+                    if grad.is_sparse:
+                        raise RuntimeError("Sparse gradient is not supported")
+                    state = self.state[p]
+                    # New state: its allocations and this parameter's launch alternate, so that
+                    # the GPU works while the host allocates.  A gradient in another dtype: one
+                    # bf16 copy at a time.
+                    alone = not state or grad.dtype != torch.bfloat16 or not grad.is_cuda
+                    if due and (alone or len(due) == MANY_TENSORS or state["step"] + 1 != due[0][2]["step"]):
+                        self._step_due(group, due)
+                        if p.grad is None:  # a packed weight that the group lists twice
+                            continue
+                    self._init_state_if_empty(p, state)
+                    state["step"] += 1
+                    quant = is_quant(p)
+                    if quant:
+                        self._warn_lossy_master_once(state)
+                    tensors = {k: state[k] for k in states}
+                    tensors["grad"] = grad if grad.dtype == torch.bfloat16 else grad.to(torch.bfloat16)
+                    seed = self._rng.getrandbits(63) if with_seed else 0
+                    # a quantized weight has no bf16 image to write: only the master moves,
+                    # then copy_ re-quantizes the packed payload from it
+                    due.append((p, quant, state, (None if quant else p.data, tensors, seed)))
+                    if alone:
+                        self._step_due(group, due)
+            finally:  # an error stops at its parameter: those before it are stepped
+                self._step_due(group, due)
         return loss
 
-    def _step_pending(self, group, pending):
+    def _step_due(self, group, due):
+        items = due[:]
+        due.clear()
+        if not items:
+            return
         beta1, beta2 = group["betas"]
-        for step, items in pending.items():
-            cuda = [it for it in items if it[2]["grad"].is_cuda]
-            if cuda:
-                adam_step_many(self.mode, [(None if quant else p.data, tensors, seed) for p, quant, tensors, seed in cuda],
-                               group["lr"], group["weight_decay"], beta1, beta2, group["eps"], step,
-                               self.decoupled_weight_decay)
-            for p, quant, tensors, seed in items:
-                if not tensors["grad"].is_cuda:
-                    self.step_fn(None if quant else p.data, tensors, group["lr"], group["weight_decay"], beta1, beta2,
-                                 group["eps"], step, decoupled_weight_decay=self.decoupled_weight_decay,
-                                 **({"seed": seed} if self.mode == "stochastic_rounding" else {}))
+        step, stepped = items[0][2]["step"], 0
+        try:
+            if len(items) == 1:
+                params, tensors, seed = items[0][3]
+                self.step_fn(params, tensors, group["lr"], group["weight_decay"], beta1, beta2, group["eps"], step,
+                             decoupled_weight_decay=self.decoupled_weight_decay,
+                             **({"seed": seed} if self.mode == "stochastic_rounding" else {}))
+            else:
+                adam_step_many(self.mode, [it[3] for it in items], group["lr"], group["weight_decay"], beta1, beta2,
+                               group["eps"], step, self.decoupled_weight_decay)
+            stepped = len(items)
+        except Exception as e:
+            stepped = getattr(e, "stepped", 0)
+            for _, _, state, _ in items[stepped + 1:]:  # not reached
+                state["step"] -= 1
+            raise
+        finally:
+            for p, quant, _, (_, tensors, _) in items[:stepped]:
                 if quant:
                     p.data.copy_(tensors["master_params"])
                     p.grad = None
-        pending.clear()
 
     # ------------------------------------------------------------- checkpoint
     @torch.no_grad()

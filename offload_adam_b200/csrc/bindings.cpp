@@ -134,21 +134,29 @@ void adam_step(int64_t mode, const OptT& p, const OptT& g, const OptT& g2, const
 
 // The same step over many tensors with common hyper-parameters: lists of equal length, a
 // null parameter where only the master moves, no extra state for stochastic rounding.
-void adam_step_many(int64_t mode, const std::vector<OptT>& p, const std::vector<Tensor>& g, const std::vector<Tensor>& m,
-                    const std::vector<Tensor>& v, const std::vector<OptT>& extra, const std::vector<int64_t>& seeds,
-                    double lr, double wd, double b1h, double b2h, double eps, bool decoupled) {
+// Returns the number of leading tensors that it stepped: all, or those before the first one
+// that adam_step refuses.
+int64_t adam_step_many(int64_t mode, const std::vector<OptT>& p, const std::vector<Tensor>& g, const std::vector<Tensor>& m,
+                       const std::vector<Tensor>& v, const std::vector<OptT>& extra, const std::vector<int64_t>& seeds,
+                       double lr, double wd, double b1h, double b2h, double eps, bool decoupled) {
   const size_t k = g.size();
   TORCH_CHECK(p.size() == k && m.size() == k && v.size() == k && extra.size() == k && seeds.size() == k,
               "adam_step_many: lists of one length");
-  std::vector<oab::ManyEntry> e(k);
-  for (size_t i = 0; i < k; ++i) {
-    const auto a = make_args(mode, p[i], OptT(g[i]), OptT(), m[i], v[i], extra[i], lr, wd, b1h, b2h, eps, decoupled,
-                             OptT(), seeds[i], 0, OptT(), 0);
-    e[i] = {a.p, a.g, a.m, a.v, a.extra, a.n, a.seed, 0, 0};
+  std::vector<oab::ManyEntry> e;
+  e.reserve(k);
+  try {
+    for (size_t i = 0; i < k; ++i) {
+      const auto a = make_args(mode, p[i], OptT(g[i]), OptT(), m[i], v[i], extra[i], lr, wd, b1h, b2h, eps, decoupled,
+                               OptT(), seeds[i], 0, OptT(), 0);
+      if (a.g == nullptr) break;  // an empty gradient
+      e.push_back({a.p, a.g, a.m, a.v, a.extra, a.n, a.seed, 0, 0});
+    }
+  } catch (const c10::Error&) {  // tensor e.size() is refused
   }
-  cu_check(oab::launch_adam_step_many(e.data(), (int)k, (int)mode, decoupled, (float)lr, (float)wd, (float)b1h, (float)b2h,
-                                      (float)eps, pick_stream(0)),
+  cu_check(oab::launch_adam_step_many(e.data(), (int)e.size(), (int)mode, decoupled, (float)lr, (float)wd, (float)b1h,
+                                      (float)b2h, (float)eps, pick_stream(0)),
            "adam_step_many launch");
+  return (int64_t)e.size();
 }
 
 void grad_accumulate(const OptT& out, const Tensor& a, const OptT& b, const OptT& sumsq,

@@ -87,18 +87,31 @@ def adam_step(
         )
 
 
+MANY_TENSORS = 120  # tensors per launch of adam_step_many (csrc/adam_step.h kManyTensors)
+
+
 def adam_step_many(mode, items, lr, weight_decay, beta1, beta2, eps, step, decoupled_weight_decay=False):
-    """One launch (per 120 tensors) for ``items``, a list of ``(params or None, states, seed)``
-    of CUDA tensors that share hyper-parameters and step count; the same bits as
-    :func:`adam_step` tensor by tensor."""
+    """One launch (per ``MANY_TENSORS`` tensors) for ``items``, a list of
+    ``(params or None, states, seed)`` of CUDA tensors that share hyper-parameters and step
+    count; the same bits as :func:`adam_step` tensor by tensor.  A tensor that
+    :func:`adam_step` refuses ends the step there too: those before it are stepped, and the
+    exception's ``stepped`` says how many."""
     mode_id = MODE_IDS[mode] if isinstance(mode, str) else int(mode)
     extra_key = _EXTRA_KEY[mode_id]
-    _ext.load(required=True).adam_step_many(
+    stepped = _ext.load(required=True).adam_step_many(
         mode_id, [p for p, _, _ in items], [s["grad"] for _, s, _ in items], [s["exp_avg"] for _, s, _ in items],
         [s["exp_avg_sq"] for _, s, _ in items], [s[extra_key] if extra_key else None for _, s, _ in items],
         [seed & ((1 << 63) - 1) for _, _, seed in items], float(lr), float(weight_decay), beta_hat(beta1, step),
         beta_hat(beta2, step), float(eps), bool(decoupled_weight_decay),
     )
+    if stepped < len(items):
+        p, states, seed = items[stepped]
+        try:
+            adam_step(mode, p, states, lr, weight_decay, beta1, beta2, eps, step, decoupled_weight_decay, seed=seed)
+        except Exception as e:
+            e.stepped = stepped
+            raise
+        raise RuntimeError(f"adam_step_many refused tensor {stepped}")
 
 
 def adam_step_stochastic_rounding(params, states, lr, weight_decay, beta1, beta2, eps, step,

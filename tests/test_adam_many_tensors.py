@@ -1,5 +1,7 @@
 """One launch over many tensors gives the bits of a launch per tensor."""
 
+import warnings
+
 import pytest
 import torch
 
@@ -7,6 +9,7 @@ from offload_adam_b200 import Adam, _ext
 from offload_adam_b200.adam import STATE_DTYPES
 from offload_adam_b200.ops.adam_step import _EXTRA_KEY, adam_step, adam_step_many
 from offload_adam_b200.ops.oracle import MODE_IDS
+from offload_adam_b200.qweight import NF4QWeight
 
 pytestmark = pytest.mark.gpu
 
@@ -98,3 +101,85 @@ def test_tensors_that_share_memory_are_stepped_in_order(mode, shared):
         assert p is None or torch.equal(p, q)
         for k in a:
             assert torch.equal(a[k], b[k])
+
+
+def _params(*sizes):
+    return [torch.nn.Parameter(torch.ones(n, device="cuda", dtype=torch.bfloat16)) for n in sizes]
+
+
+def test_an_error_stops_at_its_parameter():
+    """Those before it are stepped, those after it keep their step count."""
+    a, b, c = [torch.nn.Parameter(torch.ones(8, 4, device="cuda", dtype=torch.bfloat16)) for _ in range(3)]
+    opt = Adam([a, b, c], lr=1e-2, mode="fp32_master")
+    for p in (a, b, c):
+        p.grad = torch.ones_like(p)
+    opt.step()
+    before = a.clone(), b.clone(), c.clone()
+    b.grad = torch.ones(4, 8, device="cuda", dtype=torch.bfloat16).t()
+    with pytest.raises(RuntimeError, match="contiguous"):
+        opt.step()
+    assert [opt.state[p]["step"] for p in (a, b, c)] == [2, 2, 1]
+    assert (a < before[0]).all() and torch.equal(b, before[1]) and torch.equal(c, before[2])
+
+
+def test_an_empty_parameter_is_refused_as_in_a_launch_of_its_own():
+    ps = _params(17, 0, 5)
+    opt = Adam(ps, lr=1e-2, mode="fp31_master")
+    for p in ps:
+        p.grad = torch.ones_like(p)
+        opt._init_state_if_empty(p, opt.state[p])
+    with pytest.raises(RuntimeError, match="needs a gradient"):
+        opt.step()
+    assert (ps[0] < 1).all() and (ps[2] == 1).all() and [opt.state[p]["step"] for p in ps] == [1, 1, 0]
+
+
+def test_new_state_steps_at_once():
+    """What is allocated for a later parameter may fail; and the GPU need not wait for it."""
+    ps = _params(100, 200, 300)
+    opt = Adam(ps, lr=1e-2, mode="fp32_master")
+    init = opt._init_state_if_empty
+
+    def out_of_memory(p, state):
+        if p is ps[2]:
+            raise torch.cuda.OutOfMemoryError("planted")
+        init(p, state)
+
+    opt._init_state_if_empty = out_of_memory
+    for p in ps:
+        p.grad = torch.ones_like(p)
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        opt.step()
+    assert (ps[0] < 1).all() and (ps[1] < 1).all() and [opt.state[p]["step"] for p in ps[:2]] == [1, 1]
+    opt._init_state_if_empty = init
+    n0 = _ext.load(required=True).launch_count()
+    opt.step()
+    assert [opt.state[p]["step"] for p in ps] == [2, 2, 1]
+    assert _ext.load(required=True).launch_count() - n0 == 2  # the two that have state, and the third
+
+
+def test_one_copy_of_a_gradient_in_another_dtype_at_a_time():
+    ws = [torch.nn.Parameter(NF4QWeight.from_float(torch.randn(512, 1024, device="cuda"))) for _ in range(6)]
+    opt = Adam(ws, lr=1e-2, mode="fp32_master")
+    opt._quant_master_warned = True
+    for turn in range(2):
+        for w in ws:
+            w.grad = torch.randn(512, 1024, device="cuda")
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        opt.step()
+    assert torch.cuda.max_memory_allocated() - before <= 1.5 * 2 * 512 * 1024
+    assert all(w.grad is None for w in ws)
+
+
+def test_a_parameter_listed_twice_is_stepped_twice():
+    p, q = _params(1000, 1000)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        twice = Adam([{"params": [p, p]}], lr=1e-2, mode="fp31_master")
+    once = Adam([q], lr=1e-2, mode="fp31_master")
+    for _ in range(2):
+        p.grad, q.grad = torch.ones_like(p), torch.ones_like(q)
+        twice.step()
+        once.step()
+        once.step()
+    assert twice.state[p]["step"] == 4 and torch.equal(p, q)
