@@ -95,14 +95,22 @@ class RMSNorm(nn.Module):
         return F.rms_norm(x, (x.shape[-1],), self.weight, self.eps)
 
 
-def _has_hooks(module):
-    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
-                or module._backward_pre_hooks or nn.modules.module._has_any_global_hook())
+_FORWARD = {cls: cls.forward for cls in (RMSNorm, nn.Embedding)}
+
+
+def _bare_call(module):
+    """True when calling ``module`` runs its class's own ``forward`` and nothing else: no hook,
+    no ``forward`` put in its place on the instance or on the class, no compiled call."""
+    return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                or module._backward_pre_hooks or nn.modules.module._has_any_global_hook()
+                or "forward" in module.__dict__ or type(module).forward is not _FORWARD[type(module)]
+                or module._compiled_call_impl is not None)
 
 
 def _add_norm(x, delta, norm):
-    """``(x + delta, norm(x + delta))``, in one kernel unless somebody watches the module's calls."""
-    if type(norm) is RMSNorm and x.shape == delta.shape and norm._kernel_takes(x, delta) and not _has_hooks(norm):
+    """``(x + delta, norm(x + delta))``, in one kernel unless somebody watches or replaces the
+    module's calls."""
+    if type(norm) is RMSNorm and x.shape == delta.shape and norm._kernel_takes(x, delta) and _bare_call(norm):
         return _ext.load(required=True).add_rms_norm(x, delta, norm.weight, norm.eps)
     x = x + delta
     return x, norm(x)
@@ -132,7 +140,7 @@ def _embed(module, ids):
                 and module.padding_idx is None and module.max_norm is None
                 and not (module.scale_grad_by_freq or module.sparse)
                 and type(ids) is torch.Tensor and ids.dtype == torch.int64 and ids.device == w.device
-                and ids.numel() <= _ext.load(required=True).EMBED_MAX_TOKENS and not _has_hooks(module)):
+                and ids.numel() <= _ext.load(required=True).EMBED_MAX_TOKENS and _bare_call(module)):
             return _ext.load(required=True).embedding(w, ids)
     return module(ids)
 

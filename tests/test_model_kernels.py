@@ -5,6 +5,7 @@ import torch
 import torch.nn.functional as F
 
 from offload_adam_b200 import _ext
+from offload_adam_b200.models import llama
 from offload_adam_b200.models.llama import _apply_rope, _rope_tables, build_llama, tiny_llama
 
 pytestmark = pytest.mark.gpu
@@ -132,6 +133,28 @@ def test_hooks_on_a_norm_still_see_its_calls():
     plain, seen = model(ids), []
     model.model.layers[0].post_attention_layernorm.register_forward_hook(lambda m, i, o: seen.append(o))
     assert torch.equal(model(ids), plain) and len(seen) == 1 and seen[0].shape == (1, 9, 256)
+
+
+@pytest.mark.parametrize("where", ["instance", "class"])
+def test_replaced_forward_is_called(where, monkeypatch):
+    """As adapters do it: a norm's or the embedding's ``forward`` is put in its place."""
+    model = build_llama(tiny_llama(), device="cuda", seed=1)
+    ids = torch.randint(0, 1024, (1, 9), device="cuda")
+    seen = []
+    for module in (model.model.layers[1].post_attention_layernorm, model.model.embed_tokens):
+        cls, original = type(module), type(module).forward
+
+        def forward(self, x, original=original):
+            seen.append(type(self))
+            return original(self, x)
+
+        if where == "instance":
+            module.forward = forward.__get__(module)
+        else:
+            monkeypatch.setattr(cls, "forward", forward)
+    model(ids, labels=ids).backward()
+    norms = [c for c in seen if c is llama.RMSNorm]
+    assert len(norms) == (1 if where == "instance" else 5) and seen.count(torch.nn.Embedding) == 1
 
 
 def test_model_takes_the_torch_route_where_kernels_may_not_run():
