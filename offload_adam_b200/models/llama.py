@@ -110,7 +110,7 @@ def _bare_call(module):
 def _add_norm(x, delta, norm):
     """``(x + delta, norm(x + delta))``, in one kernel unless somebody watches or replaces the
     module's calls."""
-    if type(norm) is RMSNorm and x.shape == delta.shape and norm._kernel_takes(x, delta) and _bare_call(norm):
+    if type(norm) is RMSNorm and norm._kernel_takes(x, delta) and x.shape == delta.shape and _bare_call(norm):
         return _ext.load(required=True).add_rms_norm(x, delta, norm.weight, norm.eps)
     x = x + delta
     return x, norm(x)
