@@ -90,8 +90,9 @@ class RMSNorm(nn.Module):
                 and all(x.numel() > 0 and x.shape[-1] == cols and x.device == w.device for x in xs))
 
     def forward(self, x):
-        if self._kernel_takes(x):
-            return _ext.load(required=True).rms_norm(x, self.weight, self.eps)
+        if not torch.jit.is_scripting():
+            if self._kernel_takes(x):
+                return _ext.load(required=True).rms_norm(x, self.weight, self.eps)
         return F.rms_norm(x, (x.shape[-1],), self.weight, self.eps)
 
 
@@ -131,6 +132,17 @@ def _apply_rope(x, cos, sin):
     return x * cos + rot * sin
 
 
+def _rope_heads(q, k, cos, sin):
+    """Rotated ``(batch, seq, heads, dim)`` queries and keys, as ``(batch, heads, seq, dim)``."""
+    # heads in whole pairs of 8-value vectors, tables as _rope_for makes them
+    if (use_kernels(q, k, cos, sin) and q.shape[3] % 16 == 0 and cos.shape == sin.shape == (q.shape[1], q.shape[3])
+            and cos.is_contiguous() and sin.is_contiguous() and not (cos.requires_grad or sin.requires_grad)
+            and q.device == k.device == cos.device == sin.device):
+        q, k = _ext.load(required=True).rope(q, k, cos, sin)
+        return q.transpose(1, 2), k.transpose(1, 2)
+    return _apply_rope(q.transpose(1, 2), cos, sin), _apply_rope(k.transpose(1, 2), cos, sin)
+
+
 def _embed(module, ids):
     """``module(ids)``; a training step's dense gradient of the table comes from one kernel
     that also writes the zero rows.  Plain ``nn.Embedding`` without options, nobody watching."""
@@ -167,15 +179,11 @@ class Attention(nn.Module):
         if self.q_norm is not None:
             q, k = self.q_norm(q), self.k_norm(k)
         v = self.v_proj(x).view(B, S, self.nkv, self.hd).transpose(1, 2)
-        # heads in whole pairs of 8-value vectors, tables as _rope_for makes them
-        if (self.hd % 16 == 0 and use_kernels(q, k, cos, sin) and cos.shape == sin.shape == (S, self.hd)
-                and cos.is_contiguous() and sin.is_contiguous() and not (cos.requires_grad or sin.requires_grad)
-                and q.device == k.device == cos.device == sin.device):
-            q, k = _ext.load(required=True).rope(q, k, cos, sin)
-            q, k = q.transpose(1, 2), k.transpose(1, 2)
-        else:
+        if torch.jit.is_scripting():
             q = _apply_rope(q.transpose(1, 2), cos, sin)
             k = _apply_rope(k.transpose(1, 2), cos, sin)
+        else:
+            q, k = _rope_heads(q, k, cos, sin)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.nh != self.nkv)
         return self.o_proj(o.transpose(1, 2).reshape(B, S, self.nh * self.hd))
 
@@ -189,8 +197,9 @@ class MLP(nn.Module):
 
     def forward(self, x):
         gate, up = self.gate_proj(x), self.up_proj(x)
-        if use_kernels(gate, up) and gate.shape == up.shape and gate.device == up.device:
-            return self.down_proj(_ext.load(required=True).swiglu(gate, up))
+        if not torch.jit.is_scripting():
+            if use_kernels(gate, up) and gate.shape == up.shape and gate.device == up.device:
+                return self.down_proj(_ext.load(required=True).swiglu(gate, up))
         return self.down_proj(F.silu(gate) * up)
 
 
@@ -203,7 +212,12 @@ class DecoderLayer(nn.Module):
         self.mlp = MLP(cfg)
 
     def forward(self, x, cos, sin):
-        x, h = _add_norm(x, self.self_attn(self.input_layernorm(x), cos, sin), self.post_attention_layernorm)
+        attn = self.self_attn(self.input_layernorm(x), cos, sin)
+        if torch.jit.is_scripting():
+            x = x + attn
+            h = self.post_attention_layernorm(x)
+        else:
+            x, h = _add_norm(x, attn, self.post_attention_layernorm)
         return x + self.mlp(h)
 
 

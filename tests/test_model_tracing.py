@@ -1,6 +1,7 @@
 """Layers of the model under the tracers of PyTorch (CPU)."""
 
 import copy
+import warnings
 
 import pytest
 import torch
@@ -22,3 +23,12 @@ def _module(name):
 def test_symbolic_trace(name):
     module, args = _module(name)
     assert torch.allclose(torch.fx.symbolic_trace(copy.deepcopy(module))(*args), module(*args), atol=1e-6)
+
+
+@pytest.mark.parametrize("name", MODULES)
+def test_script(name):
+    module, args = _module(name)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")  # torch.jit.script is deprecated
+        scripted = torch.jit.script(module)
+    assert torch.allclose(scripted(*args), module(*args), atol=1e-6)
