@@ -449,6 +449,7 @@ cudaError_t launch_swiglu_grad(const void* gy, const void* g, const void* u, voi
 
 cudaError_t launch_rope(const RopeTensor& q, const RopeTensor& k, const void* cos, const void* sin, int64_t batch,
                         int64_t seq, int dim, bool transposed, cudaStream_t st) {
+  if (batch <= 0 || seq <= 0) return cudaSuccess;  // before the checks: an empty tensor has no address
   if (dim <= 0 || dim % 16 != 0 || !rope_ok(q) || !rope_ok(k) || !aligned(cos, 16) || !aligned(sin, 16))
     return cudaErrorInvalidValue;
   RopeArgs a{q, k, (const uint16_t*)cos, (const uint16_t*)sin, seq, 0, dim, dim / 16, (q.heads + k.heads) * (dim / 16)};

@@ -184,6 +184,25 @@ def test_model_takes_the_torch_route_where_kernels_may_not_run():
     assert torch.func.jvp(lambda x: model.model.layers[0].mlp(x), (_rand(3, 256),), (_rand(3, 256),))[1].isfinite().all()
 
 
+def test_model_on_an_empty_sequence():
+    model = build_llama(tiny_llama(), device="cuda", seed=1)
+    ids = torch.zeros(2, 0, dtype=torch.int64, device="cuda")
+    logits = model(ids)
+    assert logits.shape == (2, 0, 1024)
+    logits.sum().backward()
+    assert model.model.layers[0].self_attn.q_proj.weight.grad.abs().max() == 0
+
+
+def test_rope_of_an_empty_batch():
+    C = _ext.load(required=True)
+    cos, sin = (t.to(torch.bfloat16) for t in _rope_tables(8, 32, 1e4, "cuda"))
+    q, k = _rand(0, 8, 4, 32).requires_grad_(True), _rand(0, 8, 2, 32).requires_grad_(True)
+    qo, ko = C.rope(q, k, cos, sin)
+    assert qo.shape == q.shape and ko.shape == k.shape
+    (qo.sum() + ko.sum()).backward()
+    assert q.grad.shape == q.shape and k.grad.shape == k.shape
+
+
 # columns around a warp's 256; tokens around the order kernel's tile (2048) and its CTAs (64);
 # rows with none, some, more than 8 and all tokens; ids drawn from a few rows or all
 @pytest.mark.parametrize("cols", [8, 256, 264, 1000])
