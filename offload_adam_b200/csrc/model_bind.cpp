@@ -226,6 +226,7 @@ void bind_model(py::module_& m) {
     return std::make_pair(out[0], out[1]);
   });
   m.def("embedding", [](const Tensor& weight, const Tensor& ids) { return Embedding::apply(weight, ids); });
+  m.def("embed_kernel_wins", &oab::embed_kernel_wins);
   m.attr("EMBED_MAX_TOKENS") = oab::kEmbedMaxTokens;
   m.attr("NORM_MAX_COLS") = oab::kNormMaxCols;
   m.def("rope", [](const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {

@@ -44,7 +44,20 @@ int rms_norm_partials(int64_t rows, int cols);
 // g (n, cols) whose ids name it, zero for the others.  cols % 8 == 0, n <= kEmbedMaxTokens,
 // vocab < 2^31; ids outside the table are ignored.  `work`: embed_work_ints(n, vocab) ints.
 // Sums in fp32, in a fixed order.
-constexpr int64_t kEmbedMaxTokens = 32768;
+constexpr int64_t kEmbedMaxTokens = 24576;
+// Whether this beats PyTorch's gradient (fill, sort, partial sums, scatter).  Finding the
+// tokens of a row compares every token with every other; what it saves is passes over the
+// table.  Microseconds on a B200, ids uniform / skewed towards few rows, then
+// PyTorch's for the skewed ones:
+//   table           4096 tokens        12288               16384               24576
+//   1024 x 256      55 /  56, 139      114 / 138, 144      148 / 177, 150      294 / 347, 164
+//   8192 x 1024     49 /  48, 175      110 / 135, 223      141 / 174, 234      291 / 341, 268
+//   128256 x 1024   83 /  96, 255      163 / 207, 350      196 / 251, 401      355 / 439, 501
+//   32000 x 4096   108 / 134, 391      212 / 262, 762      252 / 316, 935      405 / 511, 1257
+inline bool embed_kernel_wins(int64_t n, int64_t vocab, int64_t cols) {
+  const int64_t table = vocab * cols;
+  return n <= 12288 || (n <= 16384 && table >= 8000000) || (n <= kEmbedMaxTokens && table >= 100000000);
+}
 int64_t embed_work_ints(int64_t n, int64_t vocab);
 cudaError_t launch_embed_grad(const void* g, const int64_t* ids, int64_t n, void* dw, int64_t vocab, int cols, int* work,
                               cudaStream_t st);

@@ -152,7 +152,7 @@ def _embed(module, ids):
                 and module.padding_idx is None and module.max_norm is None
                 and not (module.scale_grad_by_freq or module.sparse)
                 and type(ids) is torch.Tensor and ids.dtype == torch.int64 and ids.device == w.device
-                and ids.numel() <= _ext.load(required=True).EMBED_MAX_TOKENS and _bare_call(module)):
+                and _ext.load(required=True).embed_kernel_wins(ids.numel(), *w.shape) and _bare_call(module)):
             return _ext.load(required=True).embedding(w, ids)
     return module(ids)
 

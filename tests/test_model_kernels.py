@@ -238,3 +238,18 @@ def test_embedding_of_the_model_and_its_limits():
     assert (out[0][0].float() - out[1][0].float()).norm() <= 1e-2 * out[1][0].float().norm()
     with pytest.raises(RuntimeError):
         C.embedding(table, torch.zeros(C.EMBED_MAX_TOKENS + 1, dtype=torch.int64, device="cuda"))
+
+
+@pytest.mark.parametrize("n,vocab,cols,kernel", [(12288, 1024, 64, True), (12289, 1024, 64, False), (16384, 8000, 1000, True),
+                                                 (16385, 8000, 1000, False), (24576, 100000, 1000, True),
+                                                 (24577, 100000, 1000, False)])
+def test_embedding_gradient_takes_the_kernel_where_it_wins(n, vocab, cols, kernel):
+    C = _ext.load(required=True)
+    module = torch.nn.Embedding(vocab, cols, device="cuda", dtype=torch.bfloat16)
+    ids = torch.randint(0, vocab, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    n0 = C.launch_count()
+    llama._embed(module, ids).backward(torch.ones(n, cols, device="cuda", dtype=torch.bfloat16))
+    assert (C.launch_count() > n0) == kernel
+    counts = torch.bincount(ids, minlength=vocab)
+    # PyTorch sums in fp32 too; whole numbers up to 256 are exact in bf16
+    assert counts.max() <= 256 and torch.equal(module.weight.grad, counts.to(torch.bfloat16)[:, None].expand(-1, cols))
