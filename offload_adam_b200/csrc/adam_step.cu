@@ -23,7 +23,7 @@
 
 namespace oab {
 
-unsigned long long g_launch_count = 0;
+std::atomic<unsigned long long> g_launch_count{0};
 
 namespace {
 

@@ -8,16 +8,13 @@
 #include "adam_quant.h"
 #include "adam_step.h"
 #include "grad_ops.h"
+#include "launch_count.h"
 #include "offload_engine.h"
 #include "pinned_arena.h"
 #include "symm_ops.h"
 
 namespace py = pybind11;
 using at::Tensor;
-
-namespace oab {
-extern unsigned long long g_launch_count;
-}
 
 namespace {
 
@@ -486,7 +483,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("multi_tensor_adam", &multi_tensor_adam);
   m.def("multi_tensor_chunk", &oab::multi_tensor_chunk);
   m.def("sumsq_scratch_bytes", []() { return (int64_t)oab::kSumsqScratchBytes; });
-  m.def("launch_count", []() { return (int64_t)oab::g_launch_count; });
+  m.def("launch_count", []() { return (int64_t)oab::g_launch_count.load(); });
   m.def("reset_launch_count", []() { oab::g_launch_count = 0; });
 
   m.def("gpu_numa_node", &oab::gpu_numa_node);

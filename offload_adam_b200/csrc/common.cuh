@@ -10,14 +10,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-namespace oab {
+#include "launch_count.h"
 
-// ----------------------------------------------------------------------------
-// launch accounting: every wrapper that launches one of our kernels bumps this
-// counter so the benchmark can report how many of our launches ran in a region.
-// ----------------------------------------------------------------------------
-extern unsigned long long g_launch_count;
-inline void count_launch(unsigned long long n = 1) { g_launch_count += n; }
+namespace oab {
 
 // ----------------------------------------------------------------------------
 // bf16 <-> fp32 bit helpers

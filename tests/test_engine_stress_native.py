@@ -48,3 +48,15 @@ def test_engine_threads_are_race_free_under_tsan(tmp_path):
         pytest.skip("ThreadSanitizer cannot run on this host")
     assert "WARNING: ThreadSanitizer" not in run.stderr, run.stderr[-4000:]
     assert run.returncode == 0 and "all scenarios ok" in run.stdout, (run.stdout[-2000:], run.stderr[-2000:])
+
+
+def test_launches_of_several_threads_are_all_counted(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    exe = str(tmp_path / "launch_count")
+    src = os.path.join(HERE, "native", "launch_count.cpp")
+    proc = subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", src, "-o", exe], capture_output=True, text=True, timeout=300)
+    assert proc.returncode == 0, proc.stderr[-2000:]
+    run = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0, run.stdout
