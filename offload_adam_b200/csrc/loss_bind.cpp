@@ -33,6 +33,29 @@ void check_f32(const Tensor& t, int64_t n, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() >= n, name, ": CUDA fp32");
 }
 
+// Where the kernel leaves a label that the vocabulary does not have.  The host sees it when
+// that kernel has run: the call itself returns NaN, and the next one (its backward, or the
+// next loss) raises.  PyTorch's operations end the context with a device assertion instead,
+// which the next call that looks reports as late.
+int64_t* bad_label() {
+  static int64_t* const at = [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the first call may be captured
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "label report");
+    void* p = nullptr;
+    const cudaError_t e = cudaHostAlloc(&p, sizeof(int64_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "label report");
+    ok(e, "label report");
+    *static_cast<int64_t*>(p) = -1;
+    return static_cast<int64_t*>(p);
+  }();
+  return at;
+}
+void raise_bad_label() {
+  if (__atomic_load_n(bad_label(), __ATOMIC_RELAXED) < 0) return;
+  const int64_t label = __atomic_exchange_n(bad_label(), int64_t(-1), __ATOMIC_RELAXED);
+  TORCH_CHECK_INDEX(label < 0, "label ", std::to_string(label), " of an earlier cross-entropy is outside its vocabulary; that loss is NaN");
+}
+
 // An (n, V) bf16 view whose rows start 32-byte aligned.
 Tensor ce_logits_buffer(const Tensor& like, int64_t n, int64_t V) {
   c10::cuda::CUDAGuard guard(like.device());
@@ -46,8 +69,9 @@ void ce_stats(const Tensor& logits, const Tensor& labels, const Tensor& stats) {
   check_logits(logits, labels, "ce_stats");
   check_f32(stats, 3 * logits.size(0), "stats");
   c10::cuda::CUDAGuard guard(logits.device());
+  raise_bad_label();
   ok(oab::launch_ce_stats(logits.data_ptr(), pitch_of(logits), labels.data_ptr<int64_t>(), logits.size(0),
-                          logits.size(1), stats.data_ptr<float>(), cur()), "ce_stats");
+                          logits.size(1), stats.data_ptr<float>(), bad_label(), cur()), "ce_stats");
 }
 
 void ce_finish(const std::optional<Tensor>& row_loss, const Tensor& labels, const std::optional<Tensor>& loss, const Tensor& inv) {
@@ -79,6 +103,7 @@ void ce_grad(const Tensor& logits, const Tensor& labels, const Tensor& stats, co
     gp = g->data_ptr<float>();
   }
   c10::cuda::CUDAGuard guard(logits.device());
+  raise_bad_label();
   const float* s = stats.data_ptr<float>();
   ok(oab::launch_ce_grad(logits.data_ptr(), pitch_of(logits), labels.data_ptr<int64_t>(), n, logits.size(1), s, s + n,
                          inv.data_ptr<float>(), gp, grad.data_ptr(), cur()), "ce_grad");

@@ -49,7 +49,7 @@ __device__ __forceinline__ void join(float& m, float& s, float m2, float s2) {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
 ce_stats_kernel(const uint16_t* __restrict__ logits, int64_t pitch, const int64_t* __restrict__ labels, int64_t n,
-                int64_t V, float* __restrict__ stats) {
+                int64_t V, float* __restrict__ stats, volatile int64_t* bad_label) {
   __shared__ float sm_m[THREADS / 32], sm_s[THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t nvec = (V + 15) >> 4;
@@ -110,6 +110,7 @@ ce_stats_kernel(const uint16_t* __restrict__ logits, int64_t pitch, const int64_
         // an infinite maximum is the log-sum-exp itself
         const float lse = isinf(m) ? m : __fadd_rn(m, logf(s));
         const float picked = at < V ? bf16_bits_to_f32(x[at]) : NAN;
+        if (at >= V) *bad_label = at;
         stats[row] = m;
         stats[n + row] = at < V ? __fdiv_rn(1.0f, s) : NAN;
         stats[2 * n + row] = __fmul_rn(__fsub_rn(lse, picked), lab == kIgnore ? 0.f : 1.f);
@@ -227,16 +228,16 @@ bool ce_args_ok(const void* logits, int64_t pitch, int64_t V) {
 }  // namespace
 
 cudaError_t launch_ce_stats(const void* logits, int64_t pitch, const int64_t* labels, int64_t n, int64_t V,
-                            float* stats, cudaStream_t st) {
+                            float* stats, int64_t* bad_label, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  if (V <= 0 || !ce_args_ok(logits, pitch, V)) return cudaErrorInvalidValue;
+  if (bad_label == nullptr || V <= 0 || !ce_args_ok(logits, pitch, V)) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)(n < (int64_t(1) << 30) ? n : (int64_t(1) << 30));
   count_launch();
   // a thread should have at least one pair of vectors: short rows take small CTAs
   if (V <= 128 * 64)
-    ce_stats_kernel<128><<<grid, 128, 0, st>>>((const uint16_t*)logits, pitch, labels, n, V, stats);
+    ce_stats_kernel<128><<<grid, 128, 0, st>>>((const uint16_t*)logits, pitch, labels, n, V, stats, bad_label);
   else
-    ce_stats_kernel<512><<<grid, 512, 0, st>>>((const uint16_t*)logits, pitch, labels, n, V, stats);
+    ce_stats_kernel<512><<<grid, 512, 0, st>>>((const uint16_t*)logits, pitch, labels, n, V, stats, bad_label);
   return cudaGetLastError();
 }
 

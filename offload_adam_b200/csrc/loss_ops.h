@@ -11,9 +11,10 @@ constexpr int kCePitchAlign = 16;
 // Per row of bf16 `logits` (n rows of V values, `pitch` elements apart, base 32-byte
 // aligned, pitch % 16 == 0): stats[i] = max, stats[n + i] = 1 / sum exp(x - max),
 // stats[2n + i] = loss of the row against labels[i] (0 for labels[i] == -100; negative
-// labels otherwise count as class 0; labels >= V give NaN).
+// labels otherwise count as class 0).  A label >= V gives NaN and is written to *bad_label
+// (memory that the host reads), which is otherwise left alone.
 cudaError_t launch_ce_stats(const void* logits, int64_t pitch, const int64_t* labels, int64_t n, int64_t V,
-                            float* stats, cudaStream_t st);
+                            float* stats, int64_t* bad_label, cudaStream_t st);
 
 // inv[0] = 1 / max(1, number of labels != -100); loss[0] = inv * sum(row_loss[0..n)) when
 // row_loss is given, else only inv is written.  Fixed summation order.

@@ -145,3 +145,24 @@ def test_saved_tensors_may_move():
         moved = _run(chunked_linear_cross_entropy, h, w, labels, 128)
     for a, b in zip(plain, moved):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,chunk", [(20, 128), (300, 15)])
+def test_label_outside_the_vocabulary_is_refused(n, chunk):
+    """It is seen when the kernel has run: this call's loss is NaN, the next call raises."""
+    h, w, labels = _inputs(n, 64, 1000)
+    good = _run(chunked_linear_cross_entropy, h, w, labels, chunk)
+    bad = labels.clone()
+    bad[n // 2] = 1000
+    with torch.no_grad():
+        loss = chunked_linear_cross_entropy(h, w, bad, n)
+        assert loss.isnan()  # waits for it
+        with pytest.raises(IndexError, match="label 1000 .* outside its vocabulary"):
+            chunked_linear_cross_entropy(h, w, labels, chunk)
+    for a, b in zip(good, _run(chunked_linear_cross_entropy, h, w, labels, chunk)):
+        assert torch.equal(a, b)  # reported once
+    a = h.clone().requires_grad_(True)
+    loss = chunked_linear_cross_entropy(a, w, bad, n)
+    torch.cuda.synchronize()
+    with pytest.raises(IndexError, match="label 1000"):
+        loss.backward()
