@@ -166,3 +166,29 @@ def test_label_outside_the_vocabulary_is_refused(n, chunk):
     torch.cuda.synchronize()
     with pytest.raises(IndexError, match="label 1000"):
         loss.backward()
+
+
+def test_probabilities_keep_fp32_precision():
+    """Far below the row's maximum, where an approximate exponential is off by more, down to
+    what only a subnormal bf16 holds."""
+    C = _ext.load(required=True)
+    n, V = 512, 16384
+    x = C.ce_logits_buffer(torch.empty(0, device="cuda", dtype=torch.bfloat16), n, V)
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    x.copy_(-40 - 48 * torch.rand(n, V, device="cuda", generator=gen))
+    top = torch.rand(n, device="cuda", generator=gen).to(torch.bfloat16)  # the maximum of its row
+    x[:, 0] = top
+    labels = torch.zeros(n, dtype=torch.int64, device="cuda")
+    stats, inv = torch.empty(3 * n, device="cuda"), torch.ones((), device="cuda")
+    grad = C.ce_logits_buffer(x, n, V)
+    C.ce_stats(x, labels, stats)
+    C.ce_grad(x, labels, stats, inv, None, grad)
+    d = (x.float() - top.float()[:, None]).double()[:, 1:]  # the difference rounds to fp32 first
+    want = d.exp()  # the sum of a row is 1 to within 1e-13
+    normal = want > 1.2e-38
+    wrong = grad[:, 1:] != want.float().to(torch.bfloat16)
+    # a relative error of e changes the rounding of about e / 2^-8 of the values; e is 2^-22 here
+    assert wrong[normal].double().mean() <= 3e-4
+    tiny = ~normal
+    assert tiny.any()
+    assert ((grad[:, 1:].double() - want).abs()[tiny] <= 2.0 ** -8 * want[tiny] + 2.0 ** -133).all()

@@ -38,6 +38,17 @@ def test_swiglu(n):
     _close(b.grad, b64.grad)
 
 
+def test_swiglu_keeps_fp32_precision():
+    """Where an approximate exponential is off by more: for large negative gates."""
+    C = _ext.load(required=True)
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    g = (-40 - 46 * torch.rand(1 << 20, device="cuda", generator=gen)).to(torch.bfloat16)
+    u = (1 + torch.rand(1 << 20, device="cuda", generator=gen)).to(torch.bfloat16)
+    want = F.silu(g.double()) * u.double()
+    # three fp32 roundings and exp's: 2^-22 in all, which changes that / 2^-8 of the bf16 roundings
+    assert (C.swiglu(g, u) != want.float().to(torch.bfloat16)).double().mean() <= 3e-4
+
+
 def test_swiglu_views_and_second_derivative():
     C = _ext.load(required=True)
     base = _rand(64, 70, seed=4)
