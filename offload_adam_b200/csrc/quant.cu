@@ -516,16 +516,17 @@ int grid_for(int64_t work_items, int per_sm = 8) {
     default: return cudaErrorInvalidValue;                                   \
   }
 
+namespace {
+bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+}  // namespace
+
 cudaError_t launch_absmax_partials(const void* x, int dtype, int64_t n, float* partials, cudaStream_t st) {
+  if (n >= 16 && !aligned32(x)) return cudaErrorInvalidValue;  // read in 32-byte vectors
   count_launch();
   OAB_DISPATCH_IN(dtype, absmax_partials_kernel<T><<<absmax_partials(n), kThreads, 0, st>>>((const T*)x, n, partials));
   return cudaGetLastError();
 }
 int absmax_partials(int64_t n) { return grid_for((n + 15) / 16); }
-
-namespace {
-bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
-}  // namespace
 
 cudaError_t launch_nvfp4_quantize(const void* x, int dtype, int64_t numel, const float* amax, int n_amax,
                                   uint8_t* packed, uint8_t* scales, float* global_scale, cudaStream_t st) {

@@ -49,3 +49,16 @@ def test_nvfp4_two_passes(dtype, rows, cols):
         assert torch.equal(_bits(a.reshape(b.shape)), _bits(b))
     q = NVFP4QWeight(*got, cols, dtype)
     assert torch.equal(_bits(fake_quantize(x, NVFP4QWeight)), _bits(q.dequantize(dtype)))
+
+
+def test_misaligned_source_of_nvfp4_is_refused_before_any_launch():
+    """The pass for the tensor's maximum reads 32-byte vectors, as the quantization does."""
+    x = torch.randn(64 * 64 + 1, device="cuda")[1:].view(64, 64)
+    w = NVFP4QWeight.from_float(torch.randn(64, 64, device="cuda"))
+    payload = [t.clone() for t in w._payload()]
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        w.copy_(x)
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        fake_quantize(x, NVFP4QWeight)
+    torch.cuda.synchronize()
+    assert all(torch.equal(_bits(a), _bits(b)) for a, b in zip(payload, w._payload()))
