@@ -184,10 +184,9 @@ Tensor qgemv(const Packed& w, const Tensor& x, const Tensor& bias) {
   return y;
 }
 
-// The weight as backward finds it.  The Python object is asked for its payload, as the Python
-// node does: a saved-tensor hook may have returned another weight than forward had, or a
-// dense tensor.
-Tensor dense_weight(const Tensor& weight, at::ScalarType dtype) {
+// The weight that a saved-tensor hook returned in place of forward's, another one or a dense
+// tensor: its Python object is asked for its payload, as the Python node does.
+Tensor other_weight(const Tensor& weight, at::ScalarType dtype) {
   at::NoGradGuard no_grad;
   Packed w;
   {
@@ -212,18 +211,38 @@ Tensor dense_weight(const Tensor& weight, at::ScalarType dtype) {
 }
 
 // y = x W^T + b.  `weight` is the wrapper that autograd knows; its packed tensors travel
-// beside it.  It is saved as an input is: changing it in place before backward is an error,
-// and saved-tensor hooks see it.  The products of backward are ordinary operations (they can
+// beside it.  The wrapper is saved as an input is: changing it in place before backward is an
+// error, and saved-tensor hooks see it.  The products of backward are ordinary operations (they can
 // be differentiated again).  333 tokens through 2816 x 1024 int4 with bias, forward and
 // backward, a whole call (35 us of kernels): 189 us with the Python node, 135 with this one.
 struct QLinear : torch::autograd::Function<QLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias, const Packed& w) {
     c10::cuda::CUDAGuard guard(x.device());
     ctx->save_for_backward({x, weight});
+    ctx->saved_data["weight"] = weight;  // (asking the Python object costs 10 to 20 us)
+    ctx->saved_data["packed"] = w.packed;
+    ctx->saved_data["scales"] = w.scales;
+    if (w.global_scale.defined()) ctx->saved_data["global_scale"] = w.global_scale;
+    ctx->saved_data["format"] = w.format;
+    ctx->saved_data["group"] = w.group;
     ctx->saved_data["bias"] = bias.has_value() && bias->defined();
     const Tensor b = bias.has_value() ? *bias : Tensor();
     const Tensor few = qgemv(w, x, b);
     return few.defined() ? few : at::linear(x, packed_dense(w), bias);
+  }
+  static Tensor dense_weight(AutogradContext* ctx, const Tensor& weight, at::ScalarType dtype) {
+    auto& saved = ctx->saved_data;
+    if (!weight.is_same(saved["weight"].toTensor())) return other_weight(weight, dtype);
+    Packed w;
+    w.format = saved["format"].toInt();
+    w.group = saved["group"].toInt();
+    w.packed = saved["packed"].toTensor();
+    w.scales = saved["scales"].toTensor();
+    if (w.format == oab::kQNVFP4) w.global_scale = saved["global_scale"].toTensor();
+    at::NoGradGuard no_grad;
+    c10::cuda::CUDAGuard guard(w.packed.device());
+    TORCH_CHECK(packed_ok(w, w.packed.device()), "the packed weight changed its layout between forward and backward");
+    return packed_dense(w).to(dtype);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
@@ -232,7 +251,7 @@ struct QLinear : torch::autograd::Function<QLinear> {
     c10::cuda::CUDAGuard guard(gy.device());
     const Tensor g2 = gy.reshape({-1, weight.size(0)});
     Tensor gx, gw, gb;
-    if (ctx->needs_input_grad(0)) gx = g2.mm(dense_weight(weight, gy.scalar_type())).view(x.sizes());
+    if (ctx->needs_input_grad(0)) gx = g2.mm(dense_weight(ctx, weight, gy.scalar_type())).view(x.sizes());
     if (ctx->needs_input_grad(1)) gw = g2.t().mm(x.reshape({-1, weight.size(1)}));
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) gb = g2.sum(0);
     return {gx, gw, gb, Tensor()};
