@@ -486,17 +486,21 @@ int4_fake_quant_kernel(const T* x, int64_t nchunks, int lanes_per_group, T* out)
   }
 }
 
-// One item per thread, for kernels with nothing to set up and nothing to keep from item to
-// item.  14336 x 4096 to bf16 between events, L2 cold: int8 33.3 us where a grid of 8 CTAs per
-// SM took 36.4, NVFP4 31.7 and 33.7.  The NF4 kernel fills a table per CTA and gains nothing.
-unsigned grid_flat(int64_t work_items) {
-  const int64_t want = (work_items + kThreads - 1) / kThreads, cap = int64_t(1) << 30;
-  return (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
-}
 int grid_for(int64_t work_items, int per_sm = 8) {
   int64_t want = (work_items + kThreads - 1) / kThreads;
   int cap = kNumSMs * per_sm;
   return (int)(want < 1 ? 1 : (want > cap ? cap : want));
+}
+// For kernels with nothing to set up and nothing to keep from vector to vector, `bytes` of
+// result.  A result that L2 (126 MB) does not hold next to the weight leaves faster from one
+// vector per thread: 14336 x 4096 to bf16 (117 MB) int8 30.2 us, 34.0 on 8 CTAs per SM, NVFP4
+// 27.8 and 29.3; 4096 x 16384 35.9 and 39.1, 31.7 and 34.9.  A smaller one does not: 20000 x
+// 2048 (82 MB) 21.9 and 21.6, 20.4 and 18.4; 4096 x 2048 5.6 and 5.3, 5.5 and 5.2.  (Replayed
+// from a graph, results rotating through 0.4 GB.)  The NF4 kernel fills a table per CTA.
+unsigned grid_decode(int64_t vectors, int64_t bytes) {
+  if (bytes < 96000000) return (unsigned)grid_for(vectors);
+  const int64_t want = (vectors + kThreads - 1) / kThreads, cap = int64_t(1) << 30;
+  return (unsigned)(want > cap ? cap : want);
 }
 
 }  // namespace
@@ -546,7 +550,7 @@ cudaError_t launch_nvfp4_dequantize(const uint8_t* packed, const uint8_t* scales
   if (nb <= 0) return cudaSuccess;
   if (!aligned32(out) || (reinterpret_cast<uintptr_t>(packed) & 7u)) return cudaErrorInvalidValue;
   count_launch();
-  OAB_DISPATCH_IN(dtype, nvfp4_dequantize_kernel<T><<<grid_flat(nb), kThreads, 0, st>>>(packed, scales, global_scale, nb, (T*)out));
+  OAB_DISPATCH_IN(dtype, nvfp4_dequantize_kernel<T><<<grid_decode(nb, numel * (int64_t)sizeof(T)), kThreads, 0, st>>>(packed, scales, global_scale, nb, (T*)out));
   return cudaGetLastError();
 }
 
@@ -609,7 +613,11 @@ cudaError_t launch_int8_dequantize(const int8_t* q, const void* scales, int scal
                                    int64_t in_f, void* out, cudaStream_t st) {
   if (out_f <= 0) return cudaSuccess;
   count_launch();
-  OAB_DISPATCH_SCALE(scale_dtype, int8_dequantize_kernel<S><<<grid_flat((out_f * in_f + 15) / 16), kThreads, 0, st>>>(q, (const S*)scales, out_f, in_f, (S*)out));
+  // vectors of 16, as the kernel decides; element by element, 8 CTAs per SM walk rows of any
+  // length (333 x 16388: 13.3 us, from a CTA per 4096 values 17.6)
+  const int64_t vectors = (out_f * in_f + 15) / 16;
+  const bool vec = in_f % 16 == 0 && (reinterpret_cast<uintptr_t>(q) & 15u) == 0 && aligned32(out);
+  OAB_DISPATCH_SCALE(scale_dtype, int8_dequantize_kernel<S><<<grid_decode(vectors, vec ? out_f * in_f * (int64_t)sizeof(S) : 0), kThreads, 0, st>>>(q, (const S*)scales, out_f, in_f, (S*)out));
   return cudaGetLastError();
 }
 

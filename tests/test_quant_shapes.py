@@ -62,3 +62,16 @@ def test_misaligned_source_of_nvfp4_is_refused_before_any_launch():
         fake_quantize(x, NVFP4QWeight)
     torch.cuda.synchronize()
     assert all(torch.equal(_bits(a), _bits(b)) for a, b in zip(payload, w._payload()))
+
+
+# results around 96 MB, where a thread takes one vector; rows of 16 columns and others
+@pytest.mark.parametrize("rows,cols", [(11717, 4096), (11720, 4096), (12000, 4004), (1, 16), (37, 20)])
+def test_dequantize_on_every_grid(rows, cols):
+    x = _rand(rows, cols, torch.bfloat16)
+    q, s = _quantize_int8_cuda(x, torch.bfloat16)
+    assert torch.equal(Int8QWeight(q, s).dequantize(torch.bfloat16), (q.float() * s.float().reshape(-1, 1)).to(torch.bfloat16))
+    if cols % 16 == 0:
+        w = NVFP4QWeight(*_quantize_nvfp4_cuda(x), cols, torch.bfloat16)
+        half = rows // 2 + 1  # a slice below the limit against the whole
+        part = NVFP4QWeight(w.weight_packed[:half], w.block_scale_fp8[:half], w.global_scale, cols, torch.bfloat16)
+        assert torch.equal(w.dequantize()[:half], part.dequantize())
