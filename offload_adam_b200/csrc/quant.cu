@@ -49,11 +49,21 @@ __global__ void __launch_bounds__(kThreads, 8) absmax_partials_kernel(const T* x
 }
 
 // ----------------------------------------------------------------------- NVFP4
-// The tensor's max |x| from n_amax partial maxima (or from the one value itself).
+// The tensor's max |x| from n_amax partial maxima (or from the one value itself).  (A loop of
+// one load after another took 0.4 to 0.8 us more of a call: 1000 x 4096 bf16 8.9 us, now 8.1.)
 __device__ __forceinline__ float tensor_amax(const float* amax, int n_amax, float* red) {
   if (n_amax == 1) return *amax;
-  float m = 0.f;
-  for (int i = threadIdx.x; i < n_amax; i += kThreads) m = fmaxf(m, __ldg(amax + i));
+  // all loads of the partials that absmax_partials gives (8 CTAs per SM) in flight at once
+  constexpr int kLoads = (kNumSMs * 8 + kThreads - 1) / kThreads;
+  float m = 0.f, v[kLoads];
+#pragma unroll
+  for (int k = 0; k < kLoads; ++k) {
+    const int i = threadIdx.x + k * kThreads;
+    v[k] = i < n_amax ? __ldg(amax + i) : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < kLoads; ++k) m = fmaxf(m, v[k]);
+  for (int i = threadIdx.x + kLoads * kThreads; i < n_amax; i += kThreads) m = fmaxf(m, __ldg(amax + i));
   m = block_max<kThreads>(m, red);
   if (threadIdx.x == 0) red[0] = m;
   __syncthreads();
