@@ -585,17 +585,23 @@ cudaError_t launch_nf4_dequantize(const uint8_t* packed, const float* absmax, in
   return cudaGetLastError();
 }
 
-// A CTA per row where a CTA takes a row: with 16 CTAs per SM walking the rows, 14336 x 4096
-// from fp32 took 52 us between events, now 49.
 // Rows of up to 2048 columns in whole quads: a warp each (a CTA per row would leave most of
-// its threads idle).  Longer rows in whole, aligned vectors of 16: a CTA per row on 256-bit
-// accesses.  Other rows in quads of up to 16384 columns: a CTA per row on quads.  The rest,
-// the loop that reads the row twice.
+// its threads idle).  Longer rows in whole, aligned vectors of 16: CTAs that walk the rows, or
+// from fp32 a CTA per row, on 256-bit accesses (14336 x 4096 fp32 52 and 49 us between events;
+// 4096 x 16384 bf16 55 and 57).  Other rows in quads of up to 16384 columns: a CTA per row on
+// quads.  The rest, the loop that reads the row twice; it also quantizes ragged rows of up to
+// kRaggedLoopCols columns faster, where a thread has few quads of its own (bf16, quads and
+// loop: 2052 columns 13.7 and 8.7 us, 3000 14.5 and 12.3, 4100 20.2 and 17.7, 4612 15.9 and
+// 16.7, 8196 20.1 and 25.7; to the fake grid, where the loop stores single values, 14.8 and 36.3).
+constexpr int64_t kRaggedLoopCols = 4352;
 #define OAB_INT8_LAUNCH(FAKE, Q, SC, OUT)                                                              \
   do {                                                                                                 \
     auto al = [](const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; }; \
     const bool fits = in_f % 16 == 0 && al(x, 32) && (FAKE ? al(OUT, 32) : al(Q, 16));                 \
     const bool quads = in_f % 4 == 0 && al(x, 4 * sizeof(T)) && (FAKE ? al(OUT, 4 * sizeof(T)) : al(Q, 4)); \
+    const unsigned walk = (unsigned)(out_f < (int64_t)kNumSMs * 16 ? out_f : (int64_t)kNumSMs * 16);   \
+    const unsigned per_row = (unsigned)(out_f < (int64_t(1) << 30) ? out_f : (int64_t(1) << 30));      \
+    const unsigned grid = sizeof(T) == 4 ? per_row : walk;                                             \
     const unsigned warp_grid = (unsigned)((out_f + 7) / 8 < (int64_t)kNumSMs * 8 ? (out_f + 7) / 8 : (int64_t)kNumSMs * 8); \
     if (quads && in_f <= 32 * 4 * kQuads)                                                              \
       int8_quantize_quads_kernel<T, S, FAKE, 32><<<warp_grid, kThreads, 0, st>>>((const T*)x, out_f, (int)in_f, Q, SC, OUT); \
@@ -603,16 +609,15 @@ cudaError_t launch_nf4_dequantize(const uint8_t* packed, const float* absmax, in
       int8_quantize_cached_kernel<T, S, FAKE, 1><<<grid, kThreads, 0, st>>>((const T*)x, out_f, in_f, Q, SC, OUT); \
     else if (fits && in_f <= kThreads * 16 * 4)                                                        \
       int8_quantize_cached_kernel<T, S, FAKE, 4><<<grid, kThreads, 0, st>>>((const T*)x, out_f, in_f, Q, SC, OUT); \
-    else if (quads && in_f <= kThreads * 4 * kQuads)                                                   \
-      int8_quantize_quads_kernel<T, S, FAKE, kThreads><<<grid, kThreads, 0, st>>>((const T*)x, out_f, (int)in_f, Q, SC, OUT); \
+    else if (quads && in_f <= kThreads * 4 * kQuads && (FAKE || in_f > kRaggedLoopCols))               \
+      int8_quantize_quads_kernel<T, S, FAKE, kThreads><<<per_row, kThreads, 0, st>>>((const T*)x, out_f, (int)in_f, Q, SC, OUT); \
     else                                                                                               \
-      int8_quantize_kernel<T, S, FAKE><<<grid, kThreads, 0, st>>>((const T*)x, out_f, in_f, Q, SC, OUT); \
+      int8_quantize_kernel<T, S, FAKE><<<walk, kThreads, 0, st>>>((const T*)x, out_f, in_f, Q, SC, OUT); \
   } while (0)
 
 cudaError_t launch_int8_quantize(const void* x, int dtype, int64_t out_f, int64_t in_f, int8_t* q,
                                  void* scales, int scale_dtype, cudaStream_t st) {
   if (out_f <= 0) return cudaSuccess;
-  const unsigned grid = (unsigned)(out_f < (int64_t(1) << 30) ? out_f : (int64_t(1) << 30));
   count_launch();
   OAB_DISPATCH_IN(dtype, OAB_DISPATCH_SCALE(scale_dtype,
       OAB_INT8_LAUNCH(false, q, (S*)scales, nullptr)));
@@ -690,7 +695,6 @@ cudaError_t launch_fake_quant(int format, const void* x, void* out, int dtype, i
       break;
     }
     case kQInt8: {
-      const unsigned grid = (unsigned)(out_f < (int64_t(1) << 30) ? out_f : (int64_t(1) << 30));
       OAB_DISPATCH_IN(dtype, OAB_DISPATCH_SCALE(scale_dtype,
           OAB_INT8_LAUNCH(true, nullptr, (S*)nullptr, (T*)out)));
       break;

@@ -75,3 +75,13 @@ def test_dequantize_on_every_grid(rows, cols):
         half = rows // 2 + 1  # a slice below the limit against the whole
         part = NVFP4QWeight(w.weight_packed[:half], w.block_scale_fp8[:half], w.global_scale, cols, torch.bfloat16)
         assert torch.equal(w.dequantize()[:half], part.dequantize())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(2369, 4348), (2369, 4352), (2369, 4356), (2500, 2052), (2400, 4096)])
+def test_int8_more_rows_than_one_grid(dtype, rows, cols):
+    x = _rand(rows, cols, dtype)
+    q, s = _quantize_int8_cuda(x, torch.bfloat16)
+    q_ref, s_ref = quantize_int8_per_channel(x.cpu(), scale_dtype=torch.bfloat16)
+    assert torch.equal(q.cpu(), q_ref) and torch.equal(s.cpu(), s_ref)
+    assert torch.equal(_bits(fake_quantize(x, Int8QWeight)), _bits(Int8QWeight(q, s).dequantize(dtype)))
