@@ -132,10 +132,10 @@ def _apply_rope(x, cos, sin):
     return x * cos + rot * sin
 
 
-def _rope_heads(q, k, cos, sin):
-    """Rotated ``(batch, seq, heads, dim)`` queries and keys, as ``(batch, heads, seq, dim)``."""
+def _rope_heads(q, k, cos, sin, hd):
+    """Rotated ``(batch, seq, heads, hd)`` queries and keys, as ``(batch, heads, seq, hd)``."""
     # heads in whole pairs of 8-value vectors, tables as _rope_for makes them
-    if (use_kernels(q, k, cos, sin) and q.shape[3] % 16 == 0 and cos.shape == sin.shape == (q.shape[1], q.shape[3])
+    if (hd % 16 == 0 and use_kernels(q, k, cos, sin) and cos.shape == sin.shape == (q.shape[1], hd)
             and cos.is_contiguous() and sin.is_contiguous() and not (cos.requires_grad or sin.requires_grad)
             and q.device == k.device == cos.device == sin.device):
         q, k = _ext.load(required=True).rope(q, k, cos, sin)
@@ -183,7 +183,7 @@ class Attention(nn.Module):
             q = _apply_rope(q.transpose(1, 2), cos, sin)
             k = _apply_rope(k.transpose(1, 2), cos, sin)
         else:
-            q, k = _rope_heads(q, k, cos, sin)
+            q, k = _rope_heads(q, k, cos, sin, self.hd)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.nh != self.nkv)
         return self.o_proj(o.transpose(1, 2).reshape(B, S, self.nh * self.hd))
 
@@ -275,21 +275,25 @@ def _head_logits(h, weight, out, chunk):
     kernels for unaligned operands, which may split a sum and add its parts in bf16; how many
     rows there are decides it.  Those take the caller's chunk (840 x 32003: 0.17 % off 64 bits
     for 2048 rows at a time, 0.20 % for 8192)."""
-    step = chunk if weight.shape[0] % 8 else h.shape[0]
-    for s in range(0, h.shape[0], step):
-        torch.mm(h[s:s + step], weight.T, out=out[s:s + step])
+    if weight.shape[0] % 8 == 0 or h.shape[0] <= chunk:
+        torch.mm(h, weight.T, out=out)
+        return
+    for s in range(0, h.shape[0], chunk):
+        torch.mm(h[s:s + chunk], weight.T, out=out[s:s + chunk])
 
 
-def _hidden_grad(d, weight, out, rows):
-    """``out = d @ weight``.  For the same vocabularies the sum over the words is kept in fp32
+def _hidden_grad(d, weight, rows, out=None):
+    """``d @ weight``.  For the same vocabularies the sum over the words is kept in fp32
     to its end, ``rows`` rows at a time: split sums in bf16 left 0.2 to 1 % of error (60 rows of
     32003 words, hidden 64: 0.57 %), fp32 leaves the 0.17 % of the one rounding, in the same
     time (32003 x 840, 8192 rows: 3656 us, 3645 in bf16)."""
     if d.shape[1] % 8 == 0:
-        torch.mm(d, weight, out=out)
-        return
+        return torch.mm(d, weight, out=out)
+    if out is None:
+        out = torch.empty((d.shape[0], weight.shape[1]), dtype=d.dtype, device=d.device)
     for s in range(0, d.shape[0], rows):
         out[s:s + rows] = torch.mm(d[s:s + rows], weight, out_dtype=torch.float32)
+    return out
 
 
 class _KernelLinearCE(torch.autograd.Function):
@@ -332,7 +336,7 @@ class _KernelLinearCE(torch.autograd.Function):
             row_loss[s:s + n] = st[2 * n:]
             if ctx.want_grad:
                 C.ce_grad(lo, lab, st, inv, None, lo)
-                _hidden_grad(lo, weight, gh[s:s + n], max(V // 2, 128))
+                _hidden_grad(lo, weight, max(V // 2, 128), gh[s:s + n])
                 if gw is None:  # fp32 until the last; two groups are one sum
                     gw = lo.T @ hs if N <= 2 * rows else torch.mm(lo.T, hs, out_dtype=torch.float32)
                 else:
@@ -361,8 +365,7 @@ class _KernelLinearCE(torch.autograd.Function):
             C.ce_grad(logits, labels, stats, inv, None if through else g.detach().float().contiguous(), d)
             gh = gw = None
             if ctx.needs_input_grad[0]:
-                gh = torch.empty_like(h)
-                _hidden_grad(d, weight, gh, max(V, 128))
+                gh = _hidden_grad(d, weight, max(V, 128))
             if ctx.needs_input_grad[1]:
                 gw = d.T @ h
         if through:
