@@ -586,7 +586,8 @@ cudaError_t launch_nf4_dequantize(const uint8_t* packed, const float* absmax, in
 }
 
 // Rows of up to 2048 columns in whole quads: a warp each (a CTA per row would leave most of
-// its threads idle).  Longer rows in whole, aligned vectors of 16: CTAs that walk the rows, or
+// its threads idle), unless four CTAs per SM take all of them at once and vectors fit (592 x
+// 2048 bf16 to the fake grid: quads 5.0 us, vectors 3.1; 1184 x 1024 3.9 and 4.2).  Longer rows in whole, aligned vectors of 16: CTAs that walk the rows, or
 // from fp32 a CTA per row, on 256-bit accesses (14336 x 4096 fp32 52 and 49 us between events;
 // 4096 x 16384 bf16 55 and 57).  Other rows in quads of up to 16384 columns: a CTA per row on
 // quads.  The rest, the loop that reads the row twice; it also quantizes ragged rows of up to
@@ -603,7 +604,7 @@ constexpr int64_t kRaggedLoopCols = 4352;
     const unsigned per_row = (unsigned)(out_f < (int64_t(1) << 30) ? out_f : (int64_t(1) << 30));      \
     const unsigned grid = sizeof(T) == 4 ? per_row : walk;                                             \
     const unsigned warp_grid = (unsigned)((out_f + 7) / 8 < (int64_t)kNumSMs * 8 ? (out_f + 7) / 8 : (int64_t)kNumSMs * 8); \
-    if (quads && in_f <= 32 * 4 * kQuads)                                                              \
+    if (quads && in_f <= 32 * 4 * kQuads && !(fits && out_f <= kNumSMs * 4))                           \
       int8_quantize_quads_kernel<T, S, FAKE, 32><<<warp_grid, kThreads, 0, st>>>((const T*)x, out_f, (int)in_f, Q, SC, OUT); \
     else if (fits && in_f <= kThreads * 16)                                                            \
       int8_quantize_cached_kernel<T, S, FAKE, 1><<<grid, kThreads, 0, st>>>((const T*)x, out_f, in_f, Q, SC, OUT); \

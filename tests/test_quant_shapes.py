@@ -78,8 +78,9 @@ def test_dequantize_on_every_grid(rows, cols):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,cols", [(2369, 4348), (2369, 4352), (2369, 4356), (2500, 2052), (2400, 4096)])
-def test_int8_more_rows_than_one_grid(dtype, rows, cols):
+@pytest.mark.parametrize("rows,cols", [(592, 2048), (593, 2048), (592, 16), (593, 16), (2369, 4348), (2369, 4352), (2369, 4356),
+                                       (2500, 2052), (2400, 4096)])
+def test_int8_rows_around_the_limits_of_a_grid(dtype, rows, cols):
     x = _rand(rows, cols, dtype)
     q, s = _quantize_int8_cuda(x, torch.bfloat16)
     q_ref, s_ref = quantize_int8_per_channel(x.cpu(), scale_dtype=torch.bfloat16)
