@@ -97,6 +97,7 @@ class Adam(MasterLoadingMixin, Optimizer):
         states, with_seed = self.config["states"], self.mode == "stochastic_rounding"
         for group in self.param_groups:
             due = []  # CUDA parameters of one step count, which the next launch takes
+            fresh = 0  # elements of new state among them
             try:
                 for p in group["params"]:
                     grad = p.grad
@@ -105,27 +106,32 @@ class Adam(MasterLoadingMixin, Optimizer):
                     if grad.is_sparse:
                         raise RuntimeError("Sparse gradient is not supported")
                     state = self.state[p]
-                    # New state: its allocations and this parameter's launch alternate, so that
-                    # the GPU works while the host allocates.  A gradient in another dtype: one
-                    # bf16 copy at a time.
-                    alone = not state or grad.dtype != torch.bfloat16 or not grad.is_cuda
-                    if due and (alone or len(due) == MANY_TENSORS or state["step"] + 1 != due[0][2]["step"]):
+                    bf16 = grad.dtype is torch.bfloat16
+                    # a gradient in another dtype: one bf16 copy at a time
+                    alone = not bf16 or not grad.is_cuda
+                    if due and (alone or len(due) == MANY_TENSORS or state.get("step", 0) + 1 != due[0][2]["step"]):
                         self._step_due(group, due)
+                        fresh = 0
                         if p.grad is None:  # a packed weight that the group lists twice
                             continue
-                    self._init_state_if_empty(p, state)
+                    if not state:
+                        self._init_state_if_empty(p, state)
+                        fresh += p.numel()
                     state["step"] += 1
                     quant = is_quant(p)
                     if quant:
                         self._warn_lossy_master_once(state)
                     tensors = {k: state[k] for k in states}
-                    tensors["grad"] = grad if grad.dtype == torch.bfloat16 else grad.to(torch.bfloat16)
+                    tensors["grad"] = grad if bf16 else grad.to(torch.bfloat16)
                     seed = self._rng.getrandbits(63) if with_seed else 0
                     # a quantized weight has no bf16 image to write: only the master moves,
                     # then copy_ re-quantizes the packed payload from it
                     due.append((p, quant, state, (None if quant else p.data, tensors, seed)))
-                    if alone:
+                    # a first step's allocations and launches alternate: the GPU works while the
+                    # host allocates (4 M elements are 10 us of work, about a launch's host time)
+                    if alone or fresh >= 1 << 22:
                         self._step_due(group, due)
+                        fresh = 0
             finally:  # an error stops at its parameter: those before it are stepped
                 self._step_due(group, due)
         return loss
