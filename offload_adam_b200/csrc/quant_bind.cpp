@@ -289,7 +289,6 @@ void bind_quant(py::module_& m) {
   m.def("int4_quantize", &int4_quantize);
   m.def("int4_dequantize", &int4_dequantize);
   m.def("qlinear", &qlinear);
-  m.attr("QGEMV_MAX_TOKENS") = oab::kQGemvMaxTokens;
   m.def("fake_quant", &fake_quant, py::arg("format"), py::arg("x"), py::arg("out"), py::arg("group"),
         py::arg("scale_dtype"), py::arg("amax") = py::none());
 }

@@ -58,9 +58,9 @@ class _WeightOnlyLinear(torch.autograd.Function):
 
 def _linear(input, weight, bias=None):
     """``F.linear`` on a packed weight.  bf16 activations on CUDA take a C++ autograd node
-    (``csrc/quant_bind.cpp`` ``QLinear``); up to ``QGEMV_MAX_TOKENS`` tokens it multiplies
-    with the packed words directly (``csrc/qgemv.cu``).  Everything else takes the Python
-    node above."""
+    (``csrc/quant_bind.cpp`` ``QLinear``); one to four tokens (int4: one or two, and at least
+    1024 rows) multiply with the packed words directly (``csrc/qgemv.cu``).  Everything else
+    takes the Python node above."""
     if (isinstance(weight, QWeightBase) and weight.KERNEL_FORMAT and use_kernels(input)
             and (bias is None or use_kernels(bias))):
         packed, scales = (getattr(weight, k) for k in weight.KERNEL_PAYLOAD)

@@ -5,7 +5,6 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from offload_adam_b200 import _ext
 from offload_adam_b200.qweight import Int4QWeight, Int8QWeight, NF4QWeight, NVFP4QWeight
 
 pytestmark = pytest.mark.gpu
@@ -19,6 +18,17 @@ def _case(cls, rows, cols, tokens, bias, **kw):
 
     w = torch.nn.Parameter(cls.from_float(normal(rows, cols, std=0.02), **kw), requires_grad=False)
     return w, normal(tokens, cols), normal(rows) if bias else None
+
+
+def _takes_packed_words(w, x, b=None):
+    """Whether ``F.linear`` multiplies with the packed words: no dense bf16 copy of the weight is
+    allocated (what it does allocate is smaller: the result, and x made contiguous)."""
+    with torch.no_grad():
+        F.linear(x, w, b)  # the library's workspace
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        y = F.linear(x, w, b)
+    return torch.cuda.max_memory_allocated() - before < 2 * w.shape[0] * w.shape[1], y
 
 
 def _check(w, x, b, y):
@@ -39,24 +49,22 @@ def _check(w, x, b, y):
 @pytest.mark.parametrize("tokens", [1, 2, 3, 4])
 def test_few_tokens(cls, kw, rows, cols, tokens):
     w, x, b = _case(cls, rows, cols, tokens, bias=tokens % 2 == 0, **kw)
-    C = _ext.load(required=True)
-    with torch.no_grad():
-        n0 = C.launch_count()
-        y = F.linear(x, w, b)
-        few = C.launch_count() == n0 + 1 and (cls is not Int4QWeight or (rows >= 1024 and tokens <= 2))
+    few, y = _takes_packed_words(w, x, b)
     if cls is Int4QWeight and (rows < 1024 or tokens > 2):
+        assert not few
         dense = x @ w.data.dequantize(torch.bfloat16).T  # the dense route
         assert torch.equal(y, dense if b is None else F.linear(x, w.data.dequantize(torch.bfloat16), b))
         return
-    assert few  # no de-quantization
+    assert few
     _check(w, x, b, y)
 
 
 @pytest.mark.parametrize("cls,cols", [(NVFP4QWeight, 16), (NF4QWeight, 64), (Int8QWeight, 48)])
 def test_narrow_weights(cls, cols):
     w, x, b = _case(cls, 33, cols, 4, bias=True)
-    with torch.no_grad():
-        _check(w, x.view(2, 2, cols), b, F.linear(x.view(2, 2, cols), w, b))
+    few, y = _takes_packed_words(w, x.view(2, 2, cols), b)
+    assert few
+    _check(w, x.view(2, 2, cols), b, y)
 
 
 def test_other_calls_keep_the_dense_route():
@@ -65,15 +73,17 @@ def test_other_calls_keep_the_dense_route():
     for cls, cols, tokens, kw in ((NF4QWeight, 256, 5, {}), (Int8QWeight, 36, 2, {}),
                                   (Int4QWeight, 256, 1, {"scale_dtype": torch.float32})):
         w, x, b = _case(cls, 40, cols, tokens, bias=False, **kw)
-        with torch.no_grad():
-            assert torch.equal(F.linear(x, w), x @ w.data.dequantize(torch.bfloat16).T)
+        few, y = _takes_packed_words(w, x)
+        assert not few and torch.equal(y, x @ w.data.dequantize(torch.bfloat16).T)
     w, x, b = _case(NF4QWeight, 40, 256, 2, bias=False)
     with torch.no_grad():
         assert torch.equal(F.linear(x.half(), w), x.half() @ w.data.dequantize(torch.float16).T)
         _check(w, x, None, F.linear(x.T.contiguous().T, w))          # strided
         shifted = torch.empty(513, device="cuda", dtype=torch.bfloat16)[1:].view(2, 256).copy_(x)
-        y = F.linear(shifted, w)                                     # not 32-byte aligned
-        assert torch.equal(y, x @ w.data.dequantize(torch.bfloat16).T)
+        few, y = _takes_packed_words(w, shifted)                     # not 32-byte aligned
+        assert not few and torch.equal(y, x @ w.data.dequantize(torch.bfloat16).T)
+        few, _ = _takes_packed_words(w, x.T.contiguous().T)
+        assert few
 
 
 def test_gradients_of_a_few_tokens():
