@@ -9,10 +9,10 @@
 //
 // Row-major formats (NVFP4, NF4, int8): a lane owns 16 consecutive columns of R rows per
 // step, a warp 512 columns; the next step's words are loaded before the current ones are
-// used.  The R rows share the unpacked activations.  One token through 14336 x 4096 NF4: 18 us
-// (1.8 TB/s of packed bytes), with a dense copy 46 us.  What bounds it is not the bytes but
-// the decoding: the look-ups of 58.7 M indices keep the shared-memory pipe busy for 6.5 us and
-// the issue slots 63 % of the time.
+// used.  The R rows share the unpacked activations.  One token through 14336 x 4096 NF4: 19 us
+// of GPU time (1.7 TB/s of packed bytes), with a dense copy 43 us.  What bounds it is not the
+// bytes but the decoding: the look-ups of 58.7 M indices keep the shared-memory pipe busy for
+// 6.5 us and the issue slots 63 % of the time.
 #include "qgemv.h"
 #include "quant.h"
 #include "quant_math.cuh"

@@ -587,10 +587,11 @@ cudaError_t launch_nf4_dequantize(const uint8_t* packed, const float* absmax, in
 
 // Rows of up to 2048 columns in whole quads: a warp each (a CTA per row would leave most of
 // its threads idle), unless four CTAs per SM take all of them at once and vectors fit (592 x
-// 2048 bf16 to the fake grid: quads 5.0 us, vectors 3.1; 1184 x 1024 3.9 and 4.2).  Longer rows in whole, aligned vectors of 16: CTAs that walk the rows, or
-// from fp32 a CTA per row, on 256-bit accesses (14336 x 4096 fp32 52 and 49 us between events;
-// 4096 x 16384 bf16 55 and 57).  Other rows in quads of up to 16384 columns: a CTA per row on
-// quads.  The rest, the loop that reads the row twice; it also quantizes ragged rows of up to
+// 2048 bf16 to the fake grid: quads 5.0 us, vectors 3.1; 1184 x 1024 3.9 and 4.2).  Longer rows
+// in whole, aligned vectors of 16: CTAs that walk the rows, or from fp32 a CTA per row, on
+// 256-bit accesses (14336 x 4096 fp32 52 and 49 us between events; 4096 x 16384 bf16 55 and 57).
+// Other rows in quads of up to 16384 columns: a CTA per row on quads.  The rest, the loop that
+// reads the row twice; it also quantizes ragged rows of up to
 // kRaggedLoopCols columns faster, where a thread has few quads of its own (bf16, quads and
 // loop: 2052 columns 13.7 and 8.7 us, 3000 14.5 and 12.3, 4100 20.2 and 17.7, 4612 15.9 and
 // 16.7, 8196 20.1 and 25.7; to the fake grid, where the loop stores single values, 14.8 and 36.3).
