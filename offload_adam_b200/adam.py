@@ -144,8 +144,8 @@ class Adam(MasterLoadingMixin, Optimizer):
         beta1, beta2 = group["betas"]
         step, stepped = items[0][2]["step"], 0
         try:
-            if len(items) == 1:
-                params, tensors, seed = items[0][3]
+            params, tensors, seed = items[0][3]
+            if not tensors["grad"].is_cuda:  # one at a time
                 self.step_fn(params, tensors, group["lr"], group["weight_decay"], beta1, beta2, group["eps"], step,
                              decoupled_weight_decay=self.decoupled_weight_decay,
                              **({"seed": seed} if self.mode == "stochastic_rounding" else {}))
